@@ -66,7 +66,8 @@ typedef struct dtc_options {
   int64_t max_it;          /* CG iteration cap per load case (-ksp_max_it, :32); for the mixed
                               path the cap on the summed inner iterations */
   double inner_rtol;       /* mixed path: reduction asked of each FP32 inner solve
-                              (0 -> max(0.3 rtol, 1e-7)) */
+                              (0 -> max(0.3 rtol, 1e-7)); with inner_precond = 2 of the natural
+                              norm sqrt(r . V r), V the V-cycle */
   int32_t max_refine;      /* mixed path: cap on FP64 refinement steps (0 -> 12) */
   int32_t rotation_search; /* 1: run the CR1/CR2 rotation search (mod_struct_calcmat.f90:533-1603) */
   int32_t device;          /* CUDA device ordinal */
@@ -88,7 +89,8 @@ typedef struct dtc_options {
   int32_t inner_precond;   /* preconditioner of the FP32 inner solve: 0 = Jacobi (as PETSc's
                               PCJACOBI), 1 = node-block Jacobi (3x3 diagonal blocks),
                               2 = multigrid V-cycle on halved voxel grids (HEX20 domains are
-                              first coarsened to the HEX08 mesh of the same voxels) */
+                              first coarsened to the HEX08 mesh of the same voxels); the load
+                              cases of a domain then share one Krylov space (block CG) */
   int32_t tensor_estimator; /* how ff is formed from the solutions: 0 = projection of the
                               reaction forces (the reference, mod_struct_calcmat.f90:254-280),
                               error linear in the solve error; 1 = energy products
@@ -150,7 +152,8 @@ typedef struct dtc_domain_out {
   int64_t domain_number;
   int64_t ne, nn, nb;      /* elements, nodes, constrained nodes of the reference mesh */
   int64_t n_free_dof;      /* unconstrained DOFs the solver iterates on */
-  int64_t iters[24];       /* CG iterations per load case (summed inner iterations for mixed) */
+  int64_t iters[24];       /* CG iterations per load case (summed inner iterations for mixed; with
+                              inner_precond = 2 the load cases iterate as one block) */
   double relres[24];       /* final ||D^-1 r|| / ||D^-1 b|| evaluated in FP64 */
   double ff[576];          /* "Domain forces" ff(24,24) */
   double kmacro[576];      /* "Effective numerical stiffness" ff * vv^-1 */

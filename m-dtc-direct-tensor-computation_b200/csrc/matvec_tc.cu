@@ -123,9 +123,9 @@ int set_tc_spin_limit(long long spins, cudaStream_t s, std::string& msg) {
 // thread reads the previous round's accumulator row (tcgen05.ld: the voxel's 24 outputs),
 // scales it by the voxel's modulus factor and adds the outputs of owned nodes into shared
 // memory.  After the last round the owned active nodes get the sweep's own epilogue:
-//   kTcApply: y = scale * K u,                              acc1 += u . y  (CG: p . K p)
+//   kTcApply: y = scale * K u,                              dots += u . y unless null  (CG: p . K p)
 //   kTcRes  : y = b - K u                                   (multigrid residual)
-//   kTcPost : y = u + omega D^-1 (b - K u),  acc1 += y . y, acc2 += y . b   (post-smoothing)
+//   kTcPost : y = u + omega D^-1 (b - K u)                   (post-smoothing)
 // Precision: the split recovers FP32-level products (the tf32 rounding of the lo parts costs
 // at most 2^-21 relative); accumulation is FP32 in tensor memory, then FP64 for the scale.
 // Waits: every completion wait is bounded by g_tc_spin_limit polls; on time-out the CTA
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(128, 4)
     k_sweep_tc(const Tile* __restrict__ tiles, const DomDev* __restrict__ doms, const float* __restrict__ svox,
                const uint8_t* __restrict__ flags, const float* __restrict__ binv, const float* __restrict__ b,
                const float* __restrict__ u, float* __restrict__ y, float scale, float omega,
-               double* __restrict__ acc1, double* __restrict__ acc2, const int* __restrict__ dom_active,
+               double* __restrict__ dots, const int* __restrict__ dom_active,
                int* __restrict__ err) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char dsm[];
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(128, 4)
   }
   if (fail) return;
   // owned active interior nodes: the sweep's epilogue
-  double d1 = 0.0, d2 = 0.0;
+  double d1 = 0.0;
   for (int nl = tid >> 3; nl < 128; nl += 16) {
     const int lx = nl % kTileX, ly = (nl / kTileX) % kTileY, lz = nl / (kTileX * kTileY);
     const int x = t.x0 + lx, yv = t.y0 + ly, z = t.z0 + lz;
@@ -402,23 +402,15 @@ __global__ void __launch_bounds__(128, 4)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           v[c] = __ldg(u + k0 + c * kNLC) + dz[c];
-          d1 += (double)v[c] * (double)v[c];
-          d2 += (double)v[c] * (double)bc[c];
         }
       }
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) y[k0 + c * kNLC] = v[c];
   }
-  if (MODE == kTcApply || MODE == kTcPost) {
-    const int64_t col = (int64_t)t.dom * kNLC + lc;
+  if (MODE == kTcApply && dots) {
     const double s1 = block_sum_lc<double>(d1, red);
-    if (threadIdx.x < 8) atomicAdd(acc1 + col, s1);
-    if (MODE == kTcPost) {
-      __syncthreads();
-      const double s2 = block_sum_lc<double>(d2, red);
-      if (threadIdx.x < 8) atomicAdd(acc2 + col, s2);
-    }
+    if (threadIdx.x < 8) atomicAdd(dots + (int64_t)t.dom * kNLC + lc, s1);
   }
 }
 
@@ -431,18 +423,18 @@ int allow_sweep_tc(std::string& msg) {
 
 void launch_sweep_tc(int mode, const Tile* tiles, int64_t ntiles, const DomDev* doms, const float* svox,
                      const uint8_t* flags, const float* binv, const float* b, const float* u, float* y, float scale,
-                     float omega, double* acc1, double* acc2, const int* dom_active, int* err, cudaStream_t s) {
+                     float omega, double* dots, const int* dom_active, int* err, cudaStream_t s) {
   if (ntiles <= 0) return;
   const unsigned grid = (unsigned)(3 * ntiles);
   if (mode == kTcApply)
     k_sweep_tc<kTcApply><<<grid, 128, tc::kSweepSmem, s>>>(tiles, doms, svox, flags, binv, b, u, y, scale, omega,
-                                                            acc1, acc2, dom_active, err);
+                                                            dots, dom_active, err);
   else if (mode == kTcRes)
-    k_sweep_tc<kTcRes><<<grid, 128, tc::kSweepSmem, s>>>(tiles, doms, svox, flags, binv, b, u, y, scale, omega, acc1,
-                                                          acc2, dom_active, err);
+    k_sweep_tc<kTcRes><<<grid, 128, tc::kSweepSmem, s>>>(tiles, doms, svox, flags, binv, b, u, y, scale, omega, dots,
+                                                          dom_active, err);
   else
     k_sweep_tc<kTcPost><<<grid, 128, tc::kSweepSmem, s>>>(tiles, doms, svox, flags, binv, b, u, y, scale, omega,
-                                                           acc1, acc2, dom_active, err);
+                                                           dots, dom_active, err);
 }
 
 // Host: build the split Khat in the canonical B layout and upload it.

@@ -20,12 +20,12 @@
 // correction, so the V-cycle is a fixed SPD operator.
 //
 // One V-cycle per CG iteration, per level l that is not a domain's coarsest:
-//   t_l = omega D_l^-1 b_l                        k_mg_jacobi_flat (fine level: k_update_flat)
+//   t_l = omega D_l^-1 b_l                        k_mg_jacobi_flat (fine level: k_blk_update)
 //   r_l = b_l - K_l t_l                           k_mg_matvec<kMgRes>
 //   b_{l+1} = P^T r_l                             k_mg_restrict_flat
 //   (level l+1: recurse, or z_{l+1} = K^-1 b)     ...  / k_mg_coarse
 //   t_l += P z_{l+1}                              k_mg_prolong_flat
-//   z_l = t_l + omega D_l^-1 (b_l - K_l t_l)      k_mg_matvec<kMgPost> (+ z.z, z.b on level 0)
+//   z_l = t_l + omega D_l^-1 (b_l - K_l t_l)      k_mg_matvec<kMgPost>
 // Levels >= 2 apply the smoothing step twice before and twice after the coarse correction.
 #pragma once
 
@@ -40,24 +40,21 @@ constexpr int64_t kListNodeMask = (int64_t(1) << kListShift) - 1;
 
 // Residual / smoother on one level's interior tiles (the slab sweep of k_matvec).
 //   kMgRes : y = b - K u
-//   kMgPost: y = u + omega D^-1 (b - K u);  DOT: zz += y.y, zr += y.b per (domain, load case)
+//   kMgPost: y = u + omega D^-1 (b - K u)
 // MINB: CTAs per SM the register allocation is sized for (6: at most 80 registers; 8: 64);
 // xlen: nodes per row of the tile list (kSweepX)
-template <int MODE, bool DOT, int MINB = 6>
+template <int MODE, int MINB = 6>
 __global__ void __launch_bounds__(kThreads, MINB) k_mg_matvec(const Tile* __restrict__ tiles, const DomDev* __restrict__ doms,
                                                         const float* __restrict__ svox,
                                                         const float* __restrict__ binv, const float* __restrict__ b,
                                                         const float* __restrict__ u, float* __restrict__ y, float omega,
-                                                        double* __restrict__ acc_zz, double* __restrict__ acc_zr,
                                                         const int* __restrict__ dom_active, int xlen) {
-  __shared__ double red[32];
   const Tile t = tiles[blockIdx.x / 3];
   if (dom_active && !dom_active[t.dom]) return;
   const DomDev D = doms[t.dom];
   const int lc = (blockIdx.x % 3) * kLcGroup + (threadIdx.x & 7);
   const int row = threadIdx.x >> 3;
   const int yy = t.y0 + (row & 3), zz = t.z0 + (row >> 2);
-  double szz = 0.0, szr = 0.0;
   if (yy >= 1 && yy <= D.n[1] - 2 && zz >= 1 && zz <= D.n[2] - 2) {
     const int sy = D.n[0] * (3 * kNLC), sz = D.n[0] * D.n[1] * (3 * kNLC);
     const float* rp = u + vec_index(node_index(D, t.x0 - 1, yy, zz), 0, lc);   // plane x0 - 1
@@ -96,25 +93,9 @@ __global__ void __launch_bounds__(kThreads, MINB) k_mg_matvec(const Tile* __rest
           for (int c = 0; c < 3; ++c) v[c] = __ldg(rp + c * kNLC) + dz[c];
         }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          y[k0 + c * kNLC] = v[c];
-          if (DOT) {
-            szz += (double)v[c] * (double)v[c];
-            szr += (double)v[c] * (double)bc[c];
-          }
-        }
+        for (int c = 0; c < 3; ++c) y[k0 + c * kNLC] = v[c];
       }
       anyp = anyc;
-    }
-  }
-  if (DOT) {
-    const int64_t col = (int64_t)t.dom * kNLC + lc;
-    const double s1 = block_sum_lc<double>(szz, red);
-    __syncthreads();
-    const double s2 = block_sum_lc<double>(szr, red);
-    if (threadIdx.x < 8) {
-      atomicAdd(acc_zz + col, s1);
-      atomicAdd(acc_zr + col, s2);
     }
   }
 }
@@ -122,23 +103,19 @@ __global__ void __launch_bounds__(kThreads, MINB) k_mg_matvec(const Tile* __rest
 // Node-local second half of the residual / smoother when K t was applied by the brick kernel
 // (HEX20 fine level), z holding -K t on entry:
 //   kMgRes : z = b + z
-//   kMgPost: z = t + omega D^-1 (b + z);  DOT: zz += z.z, zr += z.b
-template <int MODE, bool DOT>
+//   kMgPost: z = t + omega D^-1 (b + z)
+template <int MODE>
 __global__ void __launch_bounds__(kThreads) k_mg_combine(const Tile* __restrict__ tiles, const DomDev* __restrict__ doms,
                                                          const uint8_t* __restrict__ flags,
                                                          const float* __restrict__ binv, const float* __restrict__ b,
                                                          const float* __restrict__ t_in, float* __restrict__ z,
-                                                         float omega, double* __restrict__ acc_zz,
-                                                         double* __restrict__ acc_zr,
-                                                         const int* __restrict__ dom_active) {
-  __shared__ double red[32];
+                                                         float omega, const int* __restrict__ dom_active) {
   const Tile t = tiles[blockIdx.x / 3];
   if (dom_active && !dom_active[t.dom]) return;
   const DomDev D = doms[t.dom];
   const int lc = (blockIdx.x % 3) * kLcGroup + (threadIdx.x & 7);
   const int row = threadIdx.x >> 3;
   const int yy = t.y0 + (row & 3), zz = t.z0 + (row >> 2);
-  double szz = 0.0, szr = 0.0;
   if (yy >= 1 && yy <= D.n[1] - 2 && zz >= 1 && zz <= D.n[2] - 2) {
     for (int i = 0; i < kTileX; ++i) {
       const int x = t.x0 + i;
@@ -162,23 +139,7 @@ __global__ void __launch_bounds__(kThreads) k_mg_combine(const Tile* __restrict_
         for (int c = 0; c < 3; ++c) v[c] = t_in[k0 + c * kNLC] + dz[c];
       }
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        z[k0 + c * kNLC] = v[c];
-        if (DOT) {
-          szz += (double)v[c] * (double)v[c];
-          szr += (double)v[c] * (double)bc[c];
-        }
-      }
-    }
-  }
-  if (DOT) {
-    const int64_t col = (int64_t)t.dom * kNLC + lc;
-    const double s1 = block_sum_lc<double>(szz, red);
-    __syncthreads();
-    const double s2 = block_sum_lc<double>(szr, red);
-    if (threadIdx.x < 8) {
-      atomicAdd(acc_zz + col, s1);
-      atomicAdd(acc_zr + col, s2);
+      for (int c = 0; c < 3; ++c) z[k0 + c * kNLC] = v[c];
     }
   }
 }
@@ -327,14 +288,10 @@ __global__ void __launch_bounds__(256) k_mg_jacobi_flat(const int64_t* __restric
 
 // Coarsest level: z = Minv b over the <= 27 interior nodes of each listed domain (one CTA per
 // domain, Minv 81 x 81 row-major on the DOFs 3 * ((x-1) + 3 (y-1) + 9 (z-1)) + c).
-// DOT (the coarsest level is the finest one): zz += z.z, zr += z.b.
-template <bool DOT>
 __global__ void __launch_bounds__(256) k_mg_coarse(const int* __restrict__ list, const DomDev* __restrict__ doms,
                                                    const float* __restrict__ minv, const float* __restrict__ b,
-                                                   float* __restrict__ z, double* __restrict__ acc_zz,
-                                                   double* __restrict__ acc_zr, const int* __restrict__ dom_active) {
+                                                   float* __restrict__ z, const int* __restrict__ dom_active) {
   __shared__ float sb[kMgDenseN * kNLC];
-  __shared__ double red[2][kNLC];
   const int d = list[blockIdx.x];
   if (dom_active && !dom_active[d]) return;
   const DomDev D = doms[d];
@@ -346,7 +303,6 @@ __global__ void __launch_bounds__(256) k_mg_coarse(const int* __restrict__ list,
     if (x < ix && y < iy && zc < iz) v = b[vec_index(node_index(D, x + 1, y + 1, zc + 1), c, lc)];
     sb[i] = v;
   }
-  if (threadIdx.x < 2 * kNLC) red[threadIdx.x / kNLC][threadIdx.x % kNLC] = 0.0;
   __syncthreads();
   const float* M = minv + (int64_t)d * kMgDenseN * kMgDenseN;
   for (int i = threadIdx.x; i < kMgDenseN * kNLC; i += blockDim.x) {
@@ -356,109 +312,7 @@ __global__ void __launch_bounds__(256) k_mg_coarse(const int* __restrict__ list,
     float s = 0.f;
     for (int k = 0; k < kMgDenseN; ++k) s = fmaf(__ldg(M + dof * kMgDenseN + k), sb[k * kNLC + lc], s);
     z[vec_index(node_index(D, x + 1, y + 1, zc + 1), c, lc)] = s;
-    if (DOT) {
-      atomicAdd(&red[0][lc], (double)s * (double)s);
-      atomicAdd(&red[1][lc], (double)s * (double)sb[dof * kNLC + lc]);
-    }
   }
-  if (DOT) {
-    __syncthreads();
-    if (threadIdx.x < kNLC) {
-      atomicAdd(acc_zz + (int64_t)d * kNLC + threadIdx.x, red[0][threadIdx.x]);
-      atomicAdd(acc_zr + (int64_t)d * kNLC + threadIdx.x, red[1][threadIdx.x]);
-    }
-  }
-}
-
-// -------------------------------------------------------------------------------------
-// Flat CG vector kernels of the multigrid path: one thread per (active interior node, 4 load
-// cases), 16-byte loads and stores, the list entry packs (domain << 40) | node.
-
-__device__ __forceinline__ void ld4(const float* p, float (&v)[4]) {
-  const float4 q = *reinterpret_cast<const float4*>(p);
-  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-}
-__device__ __forceinline__ void st4(float* p, const float (&v)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-
-// p = z + bfac p for the iterating columns (others keep p); dirf: bfac per column, NaN for a
-// column that stopped
-__global__ void __launch_bounds__(256) k_direction_flat(const int64_t* __restrict__ list, int64_t nitems,
-                                                        const float* __restrict__ z, float* __restrict__ p,
-                                                        const float* __restrict__ dirf,
-                                                        const int* __restrict__ dom_active) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nitems) return;
-  const int64_t e = __ldg(list + i / 6);
-  const int dom = (int)(e >> kListShift);
-  if (dom_active && !dom_active[dom]) return;
-  const int64_t node = e & kListNodeMask;
-  const int lc0 = 4 * (int)(i % 6);
-  float bf[4];
-  ld4(dirf + (int64_t)dom * kNLC + lc0, bf);
-  bool on[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) on[j] = !isnan(bf[j]);
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const int64_t k = (node * 3 + c) * kNLC + lc0;
-    float zv[4], pv[4];
-    ld4(z + k, zv);
-    ld4(p + k, pv);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) pv[j] = on[j] ? zv[j] + bf[j] * pv[j] : pv[j];
-    st4(p + k, pv);
-  }
-}
-
-// x += alpha p ; r -= alpha w (alpha per column from k_alpha, 0 for the columns that stopped),
-// and t = omega D^-1 r (first step of the next V-cycle) for all four
-__global__ void __launch_bounds__(256) k_update_flat(const int64_t* __restrict__ list, int64_t nitems,
-                                                     float* __restrict__ x, float* __restrict__ r,
-                                                     const float* __restrict__ p, const float* __restrict__ w,
-                                                     const float* __restrict__ alphaf,
-                                                     const float* __restrict__ binv, float omega,
-                                                     float* __restrict__ t_out, const int* __restrict__ dom_active) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nitems) return;
-  const int64_t e = __ldg(list + i / 6);
-  const int dom = (int)(e >> kListShift);
-  if (dom_active && !dom_active[dom]) return;
-  const int64_t node = e & kListNodeMask;
-  const int lc0 = 4 * (int)(i % 6);
-  float a[4];
-  ld4(alphaf + (int64_t)dom * kNLC + lc0, a);
-  float rn[3][4];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const int64_t k = (node * 3 + c) * kNLC + lc0;
-    float xv[4], pv[4], wv[4];
-    ld4(x + k, xv);
-    ld4(r + k, rn[c]);
-    ld4(p + k, pv);
-    ld4(w + k, wv);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      xv[j] = xv[j] + a[j] * pv[j];
-      rn[c][j] = rn[c][j] - a[j] * wv[j];
-    }
-    st4(x + k, xv);
-    st4(r + k, rn[c]);
-  }
-  const float2* bq = reinterpret_cast<const float2*>(binv + node * 6);   // 8-byte aligned
-  const float2 q0 = __ldg(bq), q1 = __ldg(bq + 1), q2 = __ldg(bq + 2);
-  const float b0 = q0.x, b1 = q0.y, b2 = q1.x, b3 = q1.y, b4 = q2.x, b5 = q2.y;
-  float tv[3][4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float r0 = rn[0][j], r1 = rn[1][j], r2 = rn[2][j];
-    tv[0][j] = omega * (b0 * r0 + b3 * r1 + b4 * r2);
-    tv[1][j] = omega * (b3 * r0 + b1 * r1 + b5 * r2);
-    tv[2][j] = omega * (b4 * r0 + b5 * r1 + b2 * r2);
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) st4(t_out + (node * 3 + c) * kNLC + lc0, tv[c]);
 }
 
 }  // namespace dtc
