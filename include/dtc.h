@@ -80,12 +80,9 @@ typedef struct dtc_options {
   int32_t mixed_matvec;    /* stiffness contraction of the FP32 inner solve: 0 = SIMT FP32,
                               1 = tcgen05 tensor cores (3xTF32 split, FP32-level accuracy),
                               2 = autotuned: multigrid solves time both kernels of the fine-level
-                              operator on the batch's own tiles and keep the faster; for the HEX08
-                              SIMT sweeps also the register budget (6 or 8 CTAs per SM) of each of
-                              the residual, post-smoothing and CG-application sweeps, and for
-                              every HEX08 solve that of the FP64 sweep (4 or 6 CTAs per SM);
-                              cached per device and size class (dtc_get_kernel_stats lists the
-                              timings as autotune_* classes) */
+                              operator on the batch's own tiles and keep the faster; cached per
+                              device and size class (dtc_get_kernel_stats lists the timings as
+                              autotune_* classes) */
   int32_t inner_precond;   /* preconditioner of the FP32 inner solve: 0 = Jacobi (as PETSc's
                               PCJACOBI), 1 = node-block Jacobi (3x3 diagonal blocks),
                               2 = multigrid V-cycle on halved voxel grids (HEX20 domains are

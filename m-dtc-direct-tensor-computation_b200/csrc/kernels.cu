@@ -2,9 +2,8 @@
 //
 // Operator: the assembled stiffness of the reference (MatSetValues of one Ke per element,
 // f-src/mod_dtc_main_subroutines.f90:516-579) is never formed.  HEX08: K*u is applied
-// matrix-free as a node-centric sweep: the output at node n sums, over the <= 8 kept voxels
-// around n, s_v * Khat[rows of n's corner, :] * u_v, where s_v = E_v * a and Khat the unit
-// voxel stiffness.  HEX20: element-by-element on voxel bricks staged in shared memory
+// matrix-free on voxel rows (sweep.cuh): every kept voxel adds s_v * Khat * u_v to its corners,
+// where s_v = E_v * a and Khat the unit voxel stiffness in its Hadamard basis.  HEX20: element-by-element on voxel bricks staged in shared memory
 // (ebe.cuh), nodes on the doubled grid.  Constrained DOFs (all nodes on the domain box, mod_struct_preprocess.f90:
 // 564-592) are excluded from the unknowns exactly like MatZeroRowsColumns with diag 0
 // (:945-951), so the iteration runs on the interior nodes only.
@@ -33,278 +32,15 @@
 namespace dtc {
 
 __constant__ double c_khat64[576];   // unit voxel stiffness, column-major (symmetric)
-__constant__ float c_khat32[576];
 // the 24 load-case columns of the current column pass of the macro modes for eps = 1e-6:
 // uu(nm,3,24) column-major, nm = 8 (macro order 1) or 20 (macro order 2); columns past the
 // last load case are zero
 __constant__ double c_uu[20 * 3 * kNLC];
 __constant__ double c_k20_64[3600];       // unit HEX20 element matrix (ring node order)
 
-template <typename T> struct KhatC;
-template <> struct KhatC<float> {
-  static __device__ __forceinline__ float at(int i) { return c_khat32[i]; }
-};
-template <> struct KhatC<double> {
-  static __device__ __forceinline__ double at(int i) { return c_khat64[i]; }
-};
-
-// -------------------------------------------------------------------------------------
-// HEX08: matrix-free K*u on node rows (the default SIMT operator of the corner grid).  A thread
-// owns one (y, z) row of a tile for one load case and sweeps x.  Between node planes x and x+1
-// lie the 4 voxels (x, y-1..y, z-1..z) of the row; each kept voxel contributes
-// s_v * Khat[rows of its corner, :] * u_v to node x (corner with offset 0 in x) and to node x+1
-// (offset 1), both from one read of its 8 corner values (voxel_rp / voxel_rd below).  FIRST: the
-// slab left of the tile, whose contribution to the first node only is needed.
-
-template <bool GUARD>
-__device__ __forceinline__ void load_voxels(float (&sp)[2][2], const float* __restrict__ svox, const DomDev& D, int vx,
-                                            int y, int z) {
-#pragma unroll
-  for (int b = 0; b < 2; ++b)
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int vy = y - 1 + b, vz = z - 1 + c;
-      bool ok = true;
-      if (GUARD) ok = (vx >= 0 && vx < D.L[0] && vy >= 0 && vy < D.L[1] && vz >= 0 && vz < D.L[2]);
-      const int64_t off = ok ? vx + (int64_t)D.L[0] * (vy + (int64_t)D.L[1] * vz) : 0;
-      sp[b][c] = ok ? __ldg(svox + D.vox_off + off) : 0.0f;
-    }
-}
-
-// FP32 slab on packed two-lane FMAs (sm_100 FFMA2).  A voxel of the row feeds two output rows
-// r of the thread's nodes: the corner at plane x (l0, node x) and the corner at plane x+1 (l1,
-// node x+1); one packed FMA applies both rows' entries of a column to one broadcast input value
-// (lane x: node x, lane y: node x+1), halving the FMA instructions of the scalar slab (voxel_rp).
-// The table holds the two rows' entries side by side, per voxel slot (b, c) of the row.
-__constant__ float2 c_khat32r2[4 * 3 * 24];   // [2b + c][r][col] = (Khat[3 l0 + r, col], Khat[3 l1 + r, col])
-
-// Voxel-outer FP32 slab (the FP32 sweeps): the kept voxel (b, c) of the row between planes x
-// (rp: the row's values at plane x for its load case) and x+1 reads its own 8 corners' 24 values
-// (mostly L1 hits: neighbouring rows and voxels share them) and applies them with packed FMAs.
-// No node plane stays in registers between steps, which keeps a thread at 64-80 registers (6 or
-// 8 CTAs per SM) where a window of two node planes in registers needed ~100.
-template <bool FIRST>
-__device__ __forceinline__ void voxel_rp(const float* __restrict__ rp, int sy, int sz, int b, int c, float s,
-                                         float (&cur)[3], float (&nxt)[3]) {
-  float2 acc[3];
-#pragma unroll
-  for (int r = 0; r < 3; ++r) acc[r] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int mz = 0; mz < 2; ++mz)
-#pragma unroll
-    for (int my = 0; my < 2; ++my)
-#pragma unroll
-      for (int mx = 0; mx < 2; ++mx) {
-        const int lm = corner_local(mx, my, mz);
-        const float* q = rp + mx * (3 * kNLC) + (b - 1 + my) * sy + (c - 1 + mz) * sz;
-#pragma unroll
-        for (int cj = 0; cj < 3; ++cj) {
-          const float v = __ldg(q + cj * kNLC);
-          const float2 vv = make_float2(v, v);
-#pragma unroll
-          for (int r = 0; r < 3; ++r)
-            acc[r] = __ffma2_rn(c_khat32r2[((2 * b + c) * 3 + r) * 24 + 3 * lm + cj], vv, acc[r]);
-        }
-      }
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    if (!FIRST) cur[r] = fmaf(s, acc[r].x, cur[r]);
-    nxt[r] = fmaf(s, acc[r].y, nxt[r]);
-  }
-}
-template <bool FIRST>
-__device__ __forceinline__ void row_slab(const float* __restrict__ rp, int sy, int sz, const float (&sv)[2][2],
-                                         float (&cur)[3], float (&nxt)[3]) {
-#pragma unroll
-  for (int b = 0; b < 2; ++b)
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-      if (sv[b][c] != 0.0f) voxel_rp<FIRST>(rp, sy, sz, b, c, sv[b][c], cur, nxt);
-}
-
-// Voxel-outer FP64 slab (scalar FMAs, the summation order of slab): the kept voxel (b, c) of
-// the row between planes x and x+1 reads its 8 corners' values from u, kb being the index of the
-// row's value at plane x for its load case (negative when the row starts left of the grid: a
-// voxel inside the grid has all its corners inside it, so only kept voxels' corners are read).
-template <bool FIRST>
-__device__ __forceinline__ void voxel_rd(const double* __restrict__ u, int64_t kb, int sy, int sz, int b, int c,
-                                         float s, double (&cur)[3], double (&nxt)[3]) {
-  const int l0 = corner_local(0, 1 - b, 1 - c), l1 = corner_local(1, 1 - b, 1 - c);
-  double t0 = 0, t1 = 0, t2 = 0, q0 = 0, q1 = 0, q2 = 0;
-#pragma unroll 1
-  for (int mz = 0; mz < 2; ++mz)
-#pragma unroll
-    for (int my = 0; my < 2; ++my)
-#pragma unroll
-      for (int mx = 0; mx < 2; ++mx) {
-        const int lm = corner_local(mx, my, mz);
-        const int64_t k = kb + mx * (3 * kNLC) + (b - 1 + my) * sy + (c - 1 + mz) * sz;
-#pragma unroll
-        for (int cj = 0; cj < 3; ++cj) {
-          const double v = __ldg(u + k + cj * kNLC);
-          const int col = 24 * (3 * lm + cj);
-          if (!FIRST) {
-            t0 = fma(KhatC<double>::at(col + 3 * l0 + 0), v, t0);
-            t1 = fma(KhatC<double>::at(col + 3 * l0 + 1), v, t1);
-            t2 = fma(KhatC<double>::at(col + 3 * l0 + 2), v, t2);
-          }
-          q0 = fma(KhatC<double>::at(col + 3 * l1 + 0), v, q0);
-          q1 = fma(KhatC<double>::at(col + 3 * l1 + 1), v, q1);
-          q2 = fma(KhatC<double>::at(col + 3 * l1 + 2), v, q2);
-        }
-      }
-  const double ts = (double)s;
-  if (!FIRST) {
-    cur[0] = fma(ts, t0, cur[0]);
-    cur[1] = fma(ts, t1, cur[1]);
-    cur[2] = fma(ts, t2, cur[2]);
-  }
-  nxt[0] = fma(ts, q0, nxt[0]);
-  nxt[1] = fma(ts, q1, nxt[1]);
-  nxt[2] = fma(ts, q2, nxt[2]);
-}
-template <bool FIRST>
-__device__ __forceinline__ void row_slab_d(const double* __restrict__ u, int64_t kb, int sy, int sz,
-                                           const float (&sv)[2][2], double (&cur)[3], double (&nxt)[3]) {
-#pragma unroll
-  for (int b = 0; b < 2; ++b)
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-      if (sv[b][c] != 0.0f) voxel_rd<FIRST>(u, kb, sy, sz, b, c, sv[b][c], cur, nxt);
-}
-
-
-// The 4 voxels of an interior node row between planes x and x+1 (the sweeps over interior
-// rows): a pointer that advances by one voxel per plane, 32-bit offsets of the y and z neighbours.
-struct VoxRow {
-  const float* p;
-  int sy, sz;
-  __device__ __forceinline__ void start(const float* __restrict__ svox, const DomDev& D, int vx, int y, int z) {
-    sy = D.L[0];
-    sz = D.L[0] * D.L[1];
-    p = svox + D.vox_off + vx + (int64_t)D.L[0] * ((y - 1) + (int64_t)D.L[1] * (z - 1));
-  }
-  __device__ __forceinline__ void load(float (&sp)[2][2]) const {
-#pragma unroll
-    for (int b = 0; b < 2; ++b)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) sp[b][c] = __ldg(p + b * sy + c * sz);
-  }
-};
-
-// y = scale * K u on the tile's nodes.  ALL = false: interior nodes only (inputs are
-// in-bounds without guards), optional dot accumulation acc[col] += u.y.  ALL = true: every
-// node of the grid (reaction forces; only the voxel factors need guards, since a voxel inside the
-// grid has all its corners inside it).  FP32 rows use voxel_rp, FP64 rows voxel_rd.  xlen: nodes per row of the tile list (kTileX or
-// kSweepX).  bnd_only: u vanishes off the domain box (the boundary
-// values before the first solve) and y is zero on entry; a row whose neighbour rows lie
-// inside the box then only has nonzero output at x = 1 and x = n0 - 2, and computes only those.
-// MINB: CTAs per SM the register allocation is sized for; FP32 6 (at most 80 registers) or 8 (64),
-// FP64 4 (128) or 6 (80), chosen per batch class by the sweep autotuner
-template <typename T, bool ALL, bool DOT, int MINB = (sizeof(T) == 4 ? 6 : 4)>
-__global__ void __launch_bounds__(kThreads, MINB) k_matvec(const Tile* __restrict__ tiles,
-                                                                          const DomDev* __restrict__ doms,
-                                                     const float* __restrict__ svox, const T* __restrict__ u,
-                                                     T* __restrict__ y, double scale, double* __restrict__ acc,
-                                                     const int* __restrict__ dom_active, int bnd_only, int xlen) {
-  __shared__ double red[32];
-  const Tile t = tiles[blockIdx.x / 3];
-  if (dom_active && !dom_active[t.dom]) return;
-  const DomDev D = doms[t.dom];
-  const int lc = (blockIdx.x % 3) * kLcGroup + (threadIdx.x & 7);
-  const int row = threadIdx.x >> 3;
-  const int yy = t.y0 + (row & 3), zz = t.z0 + (row >> 2);
-  const int lo = ALL ? 0 : 1;
-  const int xhi = ALL ? D.n[0] - 1 : D.n[0] - 2, yhi = ALL ? D.n[1] - 1 : D.n[1] - 2, zhi = ALL ? D.n[2] - 1 : D.n[2] - 2;
-  // nodes x0 .. xe of the row, x0 from the tile start
-  int x0 = t.x0, xe = min(xhi, t.x0 + xlen - 1);
-  if (!ALL && bnd_only && yy >= 2 && yy <= D.n[1] - 3 && zz >= 2 && zz <= D.n[2] - 3) {
-    const bool has_lo = x0 <= 1 && 1 <= xe, has_hi = x0 <= D.n[0] - 2 && D.n[0] - 2 <= xe;
-    if (has_lo && !has_hi) xe = 1;
-    else if (has_hi && !has_lo) x0 = D.n[0] - 2;
-    else if (!has_lo) xe = x0 - 1;   // neither: nothing to compute on this row
-  }
-  double dot = 0.0;
-  if constexpr (!ALL && sizeof(T) == 4) {
-    if (yy >= lo && yy <= yhi && zz >= lo && zz <= zhi && x0 <= xe) {
-      const int sy = D.n[0] * (3 * kNLC), sz = D.n[0] * D.n[1] * (3 * kNLC);
-      const float* rp = u + vec_index(node_index(D, x0 - 1, yy, zz), 0, lc);   // plane x0 - 1
-      VoxRow V;
-      float sv[2][2];
-      float cur[3] = {0.f, 0.f, 0.f}, nxt[3] = {0.f, 0.f, 0.f};
-      V.start(svox, D, x0 - 1, yy, zz);
-      V.load(sv);
-      bool anyp = (sv[0][0] != 0.f) | (sv[0][1] != 0.f) | (sv[1][0] != 0.f) | (sv[1][1] != 0.f);
-      row_slab<true>(rp, sy, sz, sv, cur, nxt);
-#pragma unroll 1
-      for (int x = x0; x <= xe; ++x) {
-        rp += 3 * kNLC;   // plane x
-        ++V.p;
-        V.load(sv);
-        const bool anyc = (sv[0][0] != 0.f) | (sv[0][1] != 0.f) | (sv[1][0] != 0.f) | (sv[1][1] != 0.f);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) { cur[c] = nxt[c]; nxt[c] = 0.f; }
-        row_slab<false>(rp, sy, sz, sv, cur, nxt);
-        if (anyp | anyc) {
-          const int64_t b = rp - u;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const float v = (float)(scale * D.scale * (double)cur[c]);
-            y[b + c * kNLC] = v;
-            if (DOT) dot += (double)__ldg(rp + c * kNLC) * (double)v;
-          }
-        }
-        anyp = anyc;
-      }
-    }
-  } else if (yy >= lo && yy <= yhi && zz >= lo && zz <= zhi && x0 <= xe) {
-    // FP64: voxel-outer slab; ALL rows may lie on the domain box, where only the voxel factors
-    // need guards (out-of-grid voxels read as void)
-    const int sy = D.n[0] * (3 * kNLC), sz = D.n[0] * D.n[1] * (3 * kNLC);
-    int64_t kx = vec_index(node_index(D, x0 - 1, yy, zz), 0, lc);   // plane x0 - 1 of the row
-    VoxRow V;
-    float sv[2][2];
-    double cur[3] = {0, 0, 0}, nxt[3] = {0, 0, 0};
-    if constexpr (ALL) {
-      load_voxels<true>(sv, svox, D, x0 - 1, yy, zz);
-    } else {
-      V.start(svox, D, x0 - 1, yy, zz);
-      V.load(sv);
-    }
-    bool anyp = (sv[0][0] != 0.f) | (sv[0][1] != 0.f) | (sv[1][0] != 0.f) | (sv[1][1] != 0.f);
-    row_slab_d<true>(u, kx, sy, sz, sv, cur, nxt);
-#pragma unroll 1
-    for (int x = x0; x <= xe; ++x) {
-      kx += 3 * kNLC;   // plane x
-      if constexpr (ALL) {
-        load_voxels<true>(sv, svox, D, x, yy, zz);
-      } else {
-        ++V.p;
-        V.load(sv);
-      }
-      const bool anyc = (sv[0][0] != 0.f) | (sv[0][1] != 0.f) | (sv[1][0] != 0.f) | (sv[1][1] != 0.f);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) { cur[c] = nxt[c]; nxt[c] = 0.0; }
-      row_slab_d<false>(u, kx, sy, sz, sv, cur, nxt);
-      if (anyp | anyc) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const double v = scale * D.scale * cur[c];
-          y[kx + c * kNLC] = v;
-          if (DOT) dot += __ldg(u + kx + c * kNLC) * v;
-        }
-      }
-      anyp = anyc;
-    }
-  }
-  if (DOT) {
-    const double s = block_sum_lc<double>(dot, red);
-    if (threadIdx.x < 8) atomicAdd(acc + (int64_t)t.dom * kNLC + lc, s);
-  }
-}
-
 }  // namespace dtc
 
+#include "sweep.cuh"
 #include "ebe.cuh"
 #include "mg.cuh"
 #include "block.cuh"
@@ -986,7 +722,7 @@ enum Buf { bDoms, bTilesI, bTilesA, bSvox, bFlags, bDinv64, bDinv32, bX, bR64, b
            bSt, bOst, bPw, bZz, bZr, bDomAct, bCount, bFf, bTarget, bErr, bBinv32, bBricksI, bBricksA, bZ32, bT32,
            bMgDoms, bMgTiles, bMgSvox, bMgFlags, bMgDinv64, bMgDinv32, bMgBinv32, bMgB, bMgT, bMgZ, bMgMinv, bMgList,
            bAdjG, bAdjV, bAdjBlk, bAdjGrad, bAdjDoms, bAdjX, bAdjSvox, bKe20, bKe20tc, bNodesI,
-           bTilesIc, bNodesIc, bBricksIc, bMgTilesC, bMgListC, bCompactCnt, bMgNodes, bMgNodesC, bXkeep, bTilesW,
+           bTilesIc, bNodesIc, bBricksIc, bMgTilesC, bMgListC, bCompactCnt, bMgNodes, bMgNodesC, bXkeep, bTilesW, bTilesWa,
            bTilesWc, bChunks, bChunksC, bNChunk, bBlkSt, bBlkCf, bGram, bGramDone, bNumBufs };
 static_assert(bNumBufs <= 80, "buffer table");
 static_assert(bSvox == 3, "DeviceSolver::Impl::svox() reads bufs[3]");
@@ -1093,32 +829,44 @@ struct Work {
   const float* ke32;
   const float* ke20tc;  // HEX20 FP32 applications on tcgen05: split matrix in the B layout, else null
   int* err;             // mbarrier time-out flag of the tensor-core kernels
-  int minb32 = 6;       // HEX08 slab sweeps: CTAs per SM of the FP32 CG application (6 or 8)
-  int minb64 = 4;       //                    and of every FP64 application (4 or 6)
-  const Tile* tw = nullptr;   // interior sweep tiles (rows of kSweepX nodes) of the slab sweeps
-  int64_t ntw = 0;
+  const Tile *tw = nullptr, *twa = nullptr;   // tiles of the HEX08 sweeps over the interior / all nodes
+  int64_t ntw = 0, ntwa = 0;
   const Chunk* chunks = nullptr;   // the node list in pieces of one domain (block CG)
   int64_t nchunks = 0;
 };
 
+// One HEX08 sweep over nt tiles.
+template <typename T, bool ALL, int MODE>
+void launch_sweep(int64_t nt, cudaStream_t s, const Tile* tiles, const DomDev* dd, const float* svox, const T* u,
+                  T* y, double scale, const float* binv, const T* b, float omega, double* acc, const int* act) {
+  if (nt <= 0) return;
+  const unsigned g = (unsigned)(nt * (kNLC / (4 * Lane<T>::kCols)));
+  k_sweep<T, ALL, MODE><<<g, kSweepThreads, kSweepSmem, s>>>(tiles, dd, svox, u, y, scale, binv, b, omega, acc, act);
+}
+
+template <typename T, bool ALL, int MODE>
+int allow_sweep_smem(std::string& msg) {
+  DTC_CUDA(cudaFuncSetAttribute(k_sweep<T, ALL, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmem));
+  return DTC_OK;
+}
+int allow_all_sweeps(std::string& msg) {
+  int e;
+  if ((e = allow_sweep_smem<float, false, kSwApply>(msg))) return e;
+  if ((e = allow_sweep_smem<float, false, kSwApplyDot>(msg))) return e;
+  if ((e = allow_sweep_smem<float, false, kSwRes>(msg))) return e;
+  if ((e = allow_sweep_smem<float, false, kSwPost>(msg))) return e;
+  if ((e = allow_sweep_smem<double, false, kSwApply>(msg))) return e;
+  if ((e = allow_sweep_smem<double, false, kSwApplyDot>(msg))) return e;
+  return allow_sweep_smem<double, true, kSwApply>(msg);
+}
+
 // y = scale * K u on the interior (ALL = false) or every node; DOT: acc[col] += u . y.
 template <typename T, int NEN, bool ALL, bool DOT>
 void apply_k(const Work& W, const DomDev* dd, const float* svox, const uint8_t* fl, const T* u, T* y, double scale,
-             double* acc, const int* act, cudaStream_t s, int bnd_only = 0) {
+             double* acc, const int* act, cudaStream_t s) {
   if constexpr (NEN == 8) {
-    // interior: the sweep tiles (rows of kSweepX nodes); every node: the node tiles
-    const int64_t nt = ALL ? W.nta : W.ntw;
-    if (nt <= 0) return;
-    const unsigned g = (unsigned)(3 * nt);
-    const Tile* tl = ALL ? W.ta : W.tw;
-    const int xl = ALL ? kTileX : kSweepX;
-    if constexpr (sizeof(T) == 4) {
-      if (W.minb32 == 8) k_matvec<T, ALL, DOT, 8><<<g, kThreads, 0, s>>>(tl, dd, svox, u, y, scale, acc, act, bnd_only, xl);
-      else k_matvec<T, ALL, DOT, 6><<<g, kThreads, 0, s>>>(tl, dd, svox, u, y, scale, acc, act, bnd_only, xl);
-    } else {
-      if (W.minb64 == 6) k_matvec<T, ALL, DOT, 6><<<g, kThreads, 0, s>>>(tl, dd, svox, u, y, scale, acc, act, bnd_only, xl);
-      else k_matvec<T, ALL, DOT, 4><<<g, kThreads, 0, s>>>(tl, dd, svox, u, y, scale, acc, act, bnd_only, xl);
-    }
+    launch_sweep<T, ALL, DOT ? kSwApplyDot : kSwApply>(ALL ? W.ntwa : W.ntw, s, ALL ? W.twa : W.tw, dd, svox, u, y,
+                                                       scale, nullptr, nullptr, 0.f, acc, act);
   } else {
     const T* ke;
     if constexpr (sizeof(T) == 8) ke = W.ke64;
@@ -1147,7 +895,7 @@ struct MgPlan {
   std::vector<DomDev> doms;                         // nlev * ndom, level-major
   std::vector<Tile> tiles;
   std::vector<int64_t> sm_off, sm_n, in_off, in_n, all_off, all_n;
-  std::vector<int64_t> sw_off, sw_n;                // smoothing tiles as rows of kSweepX nodes (slab sweeps)
+  std::vector<int64_t> sw_off, sw_n;                // smoothing tiles of the HEX08 sweeps
   std::vector<int> lists;
   std::vector<int64_t> list_off, list_n;
   std::vector<int64_t> nodes_l;                     // levels >= 1: active interior nodes, (domain << kListShift) | node
@@ -1357,9 +1105,10 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
               for (int b = 0; b < 2; ++b)
                 for (int a = 0; a < 2; ++a) act[(x + a) + (size_t)nx * ((y + b) + (size_t)ny * (z + c))] = 1;
           }
-      auto any = [&](int x0, int y0, int z0, int lo, int hx, int hy, int hz, int sx = kTileX) {
-        for (int z = std::max(z0, lo); z < std::min(z0 + kTileZ, hz + 1); ++z)
-          for (int y = std::max(y0, lo); y < std::min(y0 + kTileY, hy + 1); ++y)
+      auto any = [&](int x0, int y0, int z0, int lo, int hx, int hy, int hz, int sx = kTileX, int sy = kTileY,
+                     int sz = kTileZ) {
+        for (int z = std::max(z0, lo); z < std::min(z0 + sz, hz + 1); ++z)
+          for (int y = std::max(y0, lo); y < std::min(y0 + sy, hy + 1); ++y)
             for (int x = std::max(x0, lo); x < std::min(x0 + sx, hx + 1); ++x)
               if (act[x + (size_t)nx * (y + (size_t)ny * z)]) return true;
         return false;
@@ -1378,10 +1127,10 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
             if (any(x0, y0, z0, 0, nx - 1, ny - 1, nz - 1))
               Lv.t_all.push_back(Tile{d, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
       if (nlev[d] > l + 1)
-        for (int z0 = 1; z0 <= nz - 2; z0 += kTileZ)
-          for (int y0 = 1; y0 <= ny - 2; y0 += kTileY)
+        for (int z0 = 1; z0 <= nz - 2; z0 += kSweepZ)
+          for (int y0 = 1; y0 <= ny - 2; y0 += kSweepY)
             for (int x0 = 1; x0 <= nx - 2; x0 += kSweepX)
-              if (any(x0, y0, z0, 1, nx - 2, ny - 2, nz - 2, kSweepX))
+              if (any(x0, y0, z0, 1, nx - 2, ny - 2, nz - 2, kSweepX, kSweepY, kSweepZ))
                 Lv.t_sw.push_back(Tile{d, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
       for (int z = 1; z < nz - 1; ++z)
         for (int y = 1; y < ny - 1; ++y)
@@ -1469,18 +1218,13 @@ struct MgDev {
   const float* ke32;     // HEX20 unit element matrix (FP32)
   const float* ke20tc;   // its tensor-core operand, or null (brick SIMT kernel)
   int* err;
-  int minb_res = 6, minb_post = 6;   // HEX08 residual / post-smoothing sweeps: CTAs per SM (6 or 8)
 };
 
-// The HEX08 residual and post-smoothing sweeps with the tuned register budget (the fine
-// level's choice, used on the coarse levels too).
-// t: sweep tiles (rows of kSweepX nodes), g = 3 x their number.
+// The HEX08 residual and post-smoothing sweeps of a level over nt sweep tiles.
 template <int MODE>
-void launch_mg_matvec(int minb, unsigned g, cudaStream_t s, const Tile* t, const DomDev* d, const float* sv,
-                      const float* bi, const float* b, const float* u, float* y, float om, const int* act) {
-  if (g == 0) return;
-  if (minb == 8) k_mg_matvec<MODE, 8><<<g, kThreads, 0, s>>>(t, d, sv, bi, b, u, y, om, act, kSweepX);
-  else k_mg_matvec<MODE, 6><<<g, kThreads, 0, s>>>(t, d, sv, bi, b, u, y, om, act, kSweepX);
+void launch_mg_matvec(int64_t nt, cudaStream_t s, const Tile* t, const DomDev* d, const float* sv, const float* bi,
+                      const float* b, const float* u, float* y, float om, const int* act) {
+  launch_sweep<float, false, MODE == kMgRes ? kSwRes : kSwPost>(nt, s, t, d, sv, u, y, 1.0, bi, b, om, nullptr, act);
 }
 
 // t_ready: the fine-level t = omega D^-1 r0 was already written (by k_blk_update)
@@ -1513,8 +1257,8 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   }
   const Tile* tsm = M.tiles + P.sm_off[l];
   const unsigned g = (unsigned)(3 * nsm);
-  const Tile* tsw = M.tiles + P.sw_off[l];        // the slab sweeps' rows of kSweepX nodes
-  const unsigned gw = (unsigned)(3 * P.sw_n[l]);
+  const Tile* tsw = M.tiles + P.sw_off[l];        // the sweep tiles
+  const int64_t gw = P.sw_n[l];
   int q = -1;
   if (!(fine && t_ready)) {
     q = fine ? I.begin(0) : -1;
@@ -1533,7 +1277,7 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   float* cur = t;                  // the smoothed iterate
   float* rbuf = z;                 // the residual handed to the restriction
   if (twice) {
-    launch_mg_matvec<kMgPost>(M.minb_post, gw, s, tsw, dl, sv, bi, b, t, z, om, act);
+    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, t, z, om, act);
     ++launches;
     cur = z;
     rbuf = t;
@@ -1548,9 +1292,9 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   } else if (fine && I.tensor_matvec) {
     launch_sweep_tc(kTcRes, tsm, nsm, dl, sv, fl, bi, b, cur, rbuf, 1.0f, om, nullptr, act, M.err, s);
   } else if (fine) {
-    launch_mg_matvec<kMgRes>(M.minb_res, gw, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
+    launch_mg_matvec<kMgRes>(gw, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
   } else {
-    launch_mg_matvec<kMgRes>(M.minb_res, gw, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
+    launch_mg_matvec<kMgRes>(gw, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
   }
   if (fine) I.end(kcMgResidual, q, mb + vb, mf);          // t in, r out (mb), b in
   const DomDev* dc = M.doms + (size_t)(l + 1) * M.ndom;
@@ -1585,14 +1329,14 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   } else if (l == 0 && I.tensor_matvec)
     launch_sweep_tc(kTcPost, tsm, nsm, dl, sv, fl, bi, b, t, z, 1.0f, P.omega0, nullptr, act, M.err, s);
   else if (l == 0)
-    launch_mg_matvec<kMgPost>(M.minb_post, gw, s, tsw, dl, sv, bi, b, t, z, P.omega0, act);
+    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, t, z, P.omega0, act);
   else if (twice) {
     // z holds the corrected iterate: t = z + w D^-1 (b - K z), then z = t + w D^-1 (b - K t)
-    launch_mg_matvec<kMgPost>(M.minb_post, gw, s, tsw, dl, sv, bi, b, z, t, P.omega, act);
-    launch_mg_matvec<kMgPost>(M.minb_post, gw, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
+    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, z, t, P.omega, act);
+    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
     ++launches;
   } else
-    launch_mg_matvec<kMgPost>(M.minb_post, gw, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
+    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
   if (fine) I.end(kcMgPost, q, mb + vb + vb / 12, mf);     // t in, z out (mb), b in, D^-1
   if (!fine) I.end(kcMgCoarse, q1, 0, 0);
   launches += 2;
@@ -1928,13 +1672,11 @@ int run_cg_mg(DeviceSolver::Impl& I, int ndom, int nactive, const Work& W, const
 // DeviceSolver::prepare, which touches no device state (it may run on a host thread while the
 // solver executes an earlier pass), and consumed by DeviceSolver::solve.
 // -------------------------------------------------------------------------------------
-// Autotuner of the fine-level HEX08 sweeps (mixed_matvec = 2): the SIMT slab sweep and the
-// tcgen05 sweep run the post-smoothing step of the batch's first V-cycle on its own tiles,
-// one warm-up and three timed launches each (CUDA events on the solver stream); the faster
-// one serves the whole solve (CG operator, residual and post-smoothing sweeps share the
-// contraction).  Choices are cached per device and size class -- the median domain edge
-// (16, 24, 32, 48, 64 voxels ...) and the kept-voxel fraction (below 0.15, 0.30, above) --
-// so later batches of the same class skip the timing.
+// Autotuner of the fine-level operator (mixed_matvec = 2): the SIMT kernel and the tcgen05 kernel run on the
+// batch's own tiles, one warm-up and three timed launches each (CUDA events on the solver stream); the faster
+// one serves the whole solve.  Choices are cached per device and size class -- the median domain edge (16, 24,
+// 32, 48, 64 voxels ...) and the kept-voxel fraction (below 0.15, 0.30, above) -- so later batches of the same
+// class skip the timing.
 struct TuneKey {
   int device, nen, lclass, fclass;
   bool operator<(const TuneKey& o) const {
@@ -1943,11 +1685,7 @@ struct TuneKey {
 };
 struct TuneResult {
   int pick;            // 0 = SIMT, 1 = tensor cores
-  float ms[2];         // the timed launches of each candidate (post-smoothing; SIMT at 6 CTAs/SM)
-  // HEX08 SIMT slab sweeps: CTAs per SM of the residual, post-smoothing and CG application
-  // sweeps, and the timed launches at 6 and 8 CTAs per SM (index 0 / 1)
-  int minb[3] = {6, 6, 6};
-  float shape_ms[3][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+  float ms[2];         // the timed launches of each candidate (HEX08: the post-smoothing)
 };
 std::mutex g_tune_mu;
 std::map<TuneKey, TuneResult> g_tune_choice;
@@ -1959,13 +1697,6 @@ void record_tuning(SolverStats& st, const TuneResult& r) {
   st.kc[kcTuneSimt].ms += r.ms[0];
   st.kc[kcTuneTc].launches += kTuneReps;
   st.kc[kcTuneTc].ms += r.ms[1];
-  const int cls[3][2] = {{kcTuneRes4, kcTuneRes5}, {kcTuneSimt, kcTunePost5}, {kcTuneApply4, kcTuneApply5}};
-  for (int k = 0; k < 3; ++k)
-    for (int v = 0; v < 2; ++v)
-      if (r.shape_ms[k][v] > 0.f && !(k == 1 && v == 0)) {
-        st.kc[cls[k][v]].launches += kTuneReps;
-        st.kc[cls[k][v]].ms += r.shape_ms[k][v];
-      }
 }
 
 // CUDA-event time of kTuneReps launches after one untimed launch.
@@ -2003,9 +1734,7 @@ TuneKey tune_key(int device, int nen, const std::vector<DomDev>& doms, const std
 // The fine-level operator of an FP32 multigrid solve, chosen per device, element type and size
 // class (median domain edge in quarter octaves, kept-voxel fraction below 0.15 / 0.30 / above)
 // by CUDA-event timings on the batch's own tiles and vectors:
-//  * HEX08: the SIMT slab sweep or the tcgen05 sweep (timed on the post-smoothing sweep); for
-//    the SIMT sweep also the register budget of each of its three kernels -- residual,
-//    post-smoothing, CG application -- at 6 CTAs per SM (80 registers) or 8 (64);
+//  * HEX08: the SIMT sweep or the tcgen05 sweep (timed on the post-smoothing sweep);
 //  * HEX20: the SIMT brick kernel or the tcgen05 brick kernel (the operator of the residual and
 //    post-smoothing steps and of the CG application).
 int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, const std::vector<DomDev>& doms,
@@ -2014,9 +1743,6 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
   const TuneKey key = tune_key(I.device, nen, doms, svox);
   auto adopt = [&](const TuneResult& r) {
     I.tensor_matvec = r.pick == 1;
-    M.minb_res = r.minb[0];
-    M.minb_post = r.minb[1];
-    W.minb32 = r.minb[2];
     record_tuning(st, r);
   };
   {
@@ -2032,7 +1758,7 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
   if (nsm <= 0 || (nen == 20 && (M.nbricks0 <= 0 || !W.ke20tc))) return DTC_OK;
   const float* b = B<float>(I, bR32);
   const Tile* tsw = M.tiles + M.P->sw_off[0];
-  const unsigned gw = (unsigned)(3 * M.P->sw_n[0]);
+  const int64_t gw = M.P->sw_n[0];
   TuneResult r{0, {0.f, 0.f}};
   int e;
   for (int cand = 0; cand < 2; ++cand) {
@@ -2045,7 +1771,7 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
           launch_ebe_tc(M.bricks0, M.nbricks0, M.doms0, M.svox0, M.flags0, W.ke20tc, M.t0, M.z0, -1.0, nullptr,
                         nullptr, M.err, s);
       } else if (cand == 0) {
-        launch_mg_matvec<kMgPost>(4, gw, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
+        launch_mg_matvec<kMgPost>(gw, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
       } else {
         launch_sweep_tc(kTcPost, tsm, nsm, M.doms0, M.svox0, M.flags0, M.binv0, b, M.t0, M.z0, 1.0f, M.P->omega0,
                         nullptr, nullptr, M.err, s);
@@ -2054,71 +1780,9 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
     if ((e = time_launches(s, launch, r.ms[cand], msg))) return e;
   }
   r.pick = r.ms[1] < r.ms[0] ? 1 : 0;
-  if (nen == 8 && r.pick == 0) {
-    // register budgets of the three SIMT sweeps (the post-smoothing at 6 CTAs/SM is ms[0])
-    r.shape_ms[1][0] = r.ms[0];
-    for (int v = 0; v < 2; ++v) {
-      const int minb = v == 0 ? 6 : 8;
-      auto res = [&]() {
-        launch_mg_matvec<kMgRes>(minb, gw, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
-      };
-      if ((e = time_launches(s, res, r.shape_ms[0][v], msg))) return e;
-      if (v == 1) {
-        auto post = [&]() {
-          launch_mg_matvec<kMgPost>(minb, gw, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
-        };
-        if ((e = time_launches(s, post, r.shape_ms[1][v], msg))) return e;
-      }
-      Work Wv = W;
-      Wv.minb32 = minb;
-      auto apply = [&]() {
-        apply_k<float, 8, false, false>(Wv, M.doms0, M.svox0, M.flags0, M.t0, M.z0, 1.0, nullptr, nullptr, s);
-      };
-      if ((e = time_launches(s, apply, r.shape_ms[2][v], msg))) return e;
-    }
-    for (int k = 0; k < 3; ++k) r.minb[k] = r.shape_ms[k][1] < r.shape_ms[k][0] ? 8 : 6;
-  }
   adopt(r);
   std::lock_guard<std::mutex> lock(g_tune_mu);
   g_tune_choice[key] = r;
-  return DTC_OK;
-}
-
-// The register budget of the HEX08 FP64 slab sweep (outer residual, reactions, plain FP64 CG):
-// 4 CTAs per SM (128 registers) or 6 (80), timed on the batch's interior tiles (X -> R64, which
-// the solve overwrites next), cached per class like the FP32 choice.
-struct Tune64 { int minb; float ms[2]; };
-std::map<TuneKey, Tune64> g_tune64;
-
-int autotune_fp64(DeviceSolver::Impl& I, SolverStats& st, Work& W, const std::vector<DomDev>& doms,
-                  const std::vector<float>& svox, const double* X, double* R64, std::string& msg) {
-  const TuneKey key = tune_key(I.device, 8, doms, svox);
-  Tune64 r{4, {0.f, 0.f}};
-  bool cached = false;
-  {
-    std::lock_guard<std::mutex> lock(g_tune_mu);
-    auto it = g_tune64.find(key);
-    if (it != g_tune64.end()) { r = it->second; cached = true; }
-  }
-  if (!cached && W.nti > 0) {
-    for (int v = 0; v < 2; ++v) {
-      Work Wv = W;
-      Wv.minb64 = v == 0 ? 4 : 6;
-      auto launch = [&]() {
-        apply_k<double, 8, false, false>(Wv, B<DomDev>(I, bDoms), I.svox(), B<uint8_t>(I, bFlags), X, R64,
-                                         -1.0, nullptr, nullptr, I.stream);
-      };
-      if (int e = time_launches(I.stream, launch, r.ms[v], msg)) return e;
-    }
-    r.minb = r.ms[1] < r.ms[0] ? 6 : 4;
-    std::lock_guard<std::mutex> lock(g_tune_mu);
-    g_tune64[key] = r;
-  }
-  W.minb64 = r.minb;
-  for (int v = 0; v < 2; ++v) {
-    st.kc[v == 0 ? kcTuneF64a : kcTuneF64b].launches += kTuneReps;
-    st.kc[v == 0 ? kcTuneF64a : kcTuneF64b].ms += r.ms[v];
-  }
   return DTC_OK;
 }
 
@@ -2127,7 +1791,7 @@ struct HostBatch {
   std::vector<int64_t> tidx;   // tasks solved in this pass
   std::vector<DomDev> doms;
   std::vector<Tile> tiles_i, tiles_a, bricks_i, bricks_a;
-  std::vector<Tile> tiles_w;   // interior sweep tiles (rows of kSweepX nodes)
+  std::vector<Tile> tiles_w, tiles_wa;   // sweep tiles (HEX08) over the interior / all nodes
   std::vector<int64_t> nodes_i;
   std::vector<Chunk> chunks;   // nodes_i cut into pieces of one domain (block CG)
   std::vector<int> nchunk;     // per domain
@@ -2169,7 +1833,7 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
   // per domain: voxel factors, node activity and work lists (host threads)
   struct Packed {
     DomDev D;
-    std::vector<Tile> ti, ta, bi, ba, tw;
+    std::vector<Tile> ti, ta, bi, ba, tw, twa;
     std::vector<int64_t> ni;
     double vec = 0, mv = 0, fl = 0;
   };
@@ -2245,12 +1909,19 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
         for (int x0 = 1; x0 <= nx - 2; x0 += kTileX)
           if (any_active(x0, y0, z0, kTileX, kTileY, kTileZ, 1, nx - 2, ny - 2, nz - 2))
             out.ti.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
-    // sweep tiles (the slab sweeps over the interior): rows of kSweepX nodes
-    for (int z0 = 1; z0 <= nz - 2; z0 += kTileZ)
-      for (int y0 = 1; y0 <= ny - 2; y0 += kTileY)
-        for (int x0 = 1; x0 <= nx - 2; x0 += kSweepX)
-          if (any_active(x0, y0, z0, kSweepX, kTileY, kTileZ, 1, nx - 2, ny - 2, nz - 2))
-            out.tw.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
+    // sweep tiles (HEX08 operator) over the interior / all nodes
+    if (m == 1) {
+      for (int z0 = 1; z0 <= nz - 2; z0 += kSweepZ)
+        for (int y0 = 1; y0 <= ny - 2; y0 += kSweepY)
+          for (int x0 = 1; x0 <= nx - 2; x0 += kSweepX)
+            if (any_active(x0, y0, z0, kSweepX, kSweepY, kSweepZ, 1, nx - 2, ny - 2, nz - 2))
+              out.tw.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
+      for (int z0 = 0; z0 <= nz - 1; z0 += kSweepZ)
+        for (int y0 = 0; y0 <= ny - 1; y0 += kSweepY)
+          for (int x0 = 0; x0 <= nx - 1; x0 += kSweepX)
+            if (any_active(x0, y0, z0, kSweepX, kSweepY, kSweepZ, 0, nx - 1, ny - 1, nz - 1))
+              out.twa.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
+    }
     for (int z0 = 0; z0 <= nz - 1; z0 += kTileZ)
       for (int y0 = 0; y0 <= ny - 1; y0 += kTileY)
         for (int x0 = 0; x0 <= nx - 1; x0 += kTileX)
@@ -2284,6 +1955,7 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
     tiles_i.insert(tiles_i.end(), q.ti.begin(), q.ti.end());
     tiles_a.insert(tiles_a.end(), q.ta.begin(), q.ta.end());
     hb.tiles_w.insert(hb.tiles_w.end(), q.tw.begin(), q.tw.end());
+    hb.tiles_wa.insert(hb.tiles_wa.end(), q.twa.begin(), q.twa.end());
     bricks_i.insert(bricks_i.end(), q.bi.begin(), q.bi.end());
     bricks_a.insert(bricks_a.end(), q.ba.begin(), q.ba.end());
     nodes_i.insert(nodes_i.end(), q.ni.begin(), q.ni.end());
@@ -2313,10 +1985,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
                                              "project_f64", "mg_jacobi_f32", "mg_residual_f32",
                                              "mg_postsmooth_f32", "mg_transfer_f32", "mg_coarse_levels_f32",
                                              "rotation_search_f64", "autotune_simt_sweep", "autotune_tc_sweep",
-                                             "autotune_res_sweep_6cta", "autotune_res_sweep_8cta",
-                                             "autotune_post_sweep_8cta", "autotune_apply_sweep_6cta",
-                                             "autotune_apply_sweep_8cta", "autotune_f64_sweep_4cta",
-                                             "autotune_f64_sweep_6cta", "gram_f32", "host_pack", "host_multigrid_build"};
+                                             "gram_f32", "host_pack", "host_multigrid_build"};
   for (int c = 0; c < kcNumClasses; ++c) stats_.kc[c].name = kNames[c];
   I.stats = &stats_;
   I.profile = opt.profile_kernels != 0;
@@ -2329,20 +1998,14 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   // constant tables
   {
     double kh[576];
-    float kh32[576];
+    double wh[kWhNum];
+    float2 wh32[kWhNum];
     voxel_stiffness(8, nu, kh);
-    for (int i = 0; i < 576; ++i) kh32[i] = (float)kh[i];
+    hadamard_entries(kh, wh);
+    for (int i = 0; i < kWhNum; ++i) wh32[i] = make_float2((float)wh[i], (float)wh[i]);
     DTC_CUDA(cudaMemcpyToSymbolAsync(c_khat64, kh, sizeof(kh), 0, cudaMemcpyHostToDevice, s));
-    DTC_CUDA(cudaMemcpyToSymbolAsync(c_khat32, kh32, sizeof(kh32), 0, cudaMemcpyHostToDevice, s));
-    float2 khr[4 * 3 * 24];
-    for (int b = 0; b < 2; ++b)
-      for (int c = 0; c < 2; ++c) {
-        const int l0 = corner_local(0, 1 - b, 1 - c), l1 = corner_local(1, 1 - b, 1 - c);
-        for (int r = 0; r < 3; ++r)
-          for (int col = 0; col < 24; ++col)
-            khr[((2 * b + c) * 3 + r) * 24 + col] = make_float2(kh32[col * 24 + 3 * l0 + r], kh32[col * 24 + 3 * l1 + r]);
-      }
-    DTC_CUDA(cudaMemcpyToSymbolAsync(c_khat32r2, khr, sizeof(khr), 0, cudaMemcpyHostToDevice, s));
+    DTC_CUDA(cudaMemcpyToSymbolAsync(c_wh64, wh, sizeof(wh), 0, cudaMemcpyHostToDevice, s));
+    DTC_CUDA(cudaMemcpyToSymbolAsync(c_wh32, wh32, sizeof(wh32), 0, cudaMemcpyHostToDevice, s));
     if (int e = upload_tc_operand(kh, s, msg)) return e;
     if (I.tensor_matvec || tune) {
       if (int e = set_tc_spin_limit(opt.tc_wait_spins, s, msg)) return e;
@@ -2368,8 +2031,9 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
       }
       DTC_CUDA(cudaStreamSynchronize(s));   // the host vectors go out of scope
     }
+    if (int e = allow_all_sweeps(msg)) return e;   // per device, cheap
     if constexpr (NEN == 20)
-      if (int e = allow_all_ebe<NEN>(msg)) return e;   // per device, cheap
+      if (int e = allow_all_ebe<NEN>(msg)) return e;
   }
   // the host side of the pass (prepare_nen)
   const auto tpack = std::chrono::steady_clock::now();
@@ -2399,6 +2063,8 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   if ((e = ensure(I, bTilesA, sizeof(Tile) * std::max<int64_t>(nta, 1), msg))) return e;
   const int64_t ntw = (int64_t)hb.tiles_w.size();
   if ((e = ensure(I, bTilesW, sizeof(Tile) * std::max<int64_t>(ntw, 1), msg))) return e;
+  const int64_t ntwa = (int64_t)hb.tiles_wa.size();
+  if ((e = ensure(I, bTilesWa, sizeof(Tile) * std::max<int64_t>(ntwa, 1), msg))) return e;
   if ((e = ensure(I, bBricksI, sizeof(Tile) * std::max<int64_t>(nbi, 1), msg))) return e;
   if ((e = ensure(I, bBricksA, sizeof(Tile) * std::max<int64_t>(nba, 1), msg))) return e;
   I.svox_dev = nullptr;
@@ -2448,6 +2114,8 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   if (nta) DTC_CUDA(cudaMemcpyAsync(I.bufs[bTilesA], tiles_a.data(), sizeof(Tile) * nta, cudaMemcpyHostToDevice, s));
   if (ntw)
     DTC_CUDA(cudaMemcpyAsync(I.bufs[bTilesW], hb.tiles_w.data(), sizeof(Tile) * ntw, cudaMemcpyHostToDevice, s));
+  if (ntwa)
+    DTC_CUDA(cudaMemcpyAsync(I.bufs[bTilesWa], hb.tiles_wa.data(), sizeof(Tile) * ntwa, cudaMemcpyHostToDevice, s));
   if (nbi) DTC_CUDA(cudaMemcpyAsync(I.bufs[bBricksI], bricks_i.data(), sizeof(Tile) * nbi, cudaMemcpyHostToDevice, s));
   if ((e = ensure(I, bNodesI, sizeof(int64_t) * std::max<size_t>(nodes_i.size(), 1), msg))) return e;
   if (!nodes_i.empty())
@@ -2481,14 +2149,13 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
                ke64 ? reinterpret_cast<const float*>(ke64 + 3600) : nullptr, ke20tc, B<int>(I, bErr)};
   W.tw = B<Tile>(I, bTilesW);
   W.ntw = ntw;
+  W.twa = B<Tile>(I, bTilesWa);
+  W.ntwa = ntwa;
   const DomDev* dd = B<DomDev>(I, bDoms);
   uint8_t* fl = B<uint8_t>(I, bFlags);
   double* X = B<double>(I, bX);
   double* R64 = B<double>(I, bR64);
   int64_t& L = stats_.kernel_launches;
-  // the FP64 sweep's register budget (its cost does not depend on the values: X is zero here,
-  // R64 is scratch), before the solve's device time starts
-  if (tune && NEN == 8 && (e = autotune_fp64(I, stats_, W, doms, svox, X, R64, msg))) return e;
   DTC_CUDA(cudaEventRecord(I.ev_solve[0], s));
   if (nta) {
     DTC_CUDA(cudaMemsetAsync(I.bufs[bBinv32], 0, sizeof(float) * node_total * 6, s));
@@ -2643,7 +2310,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
       // b = -(K X)_interior with X = boundary values only (RHS of all 24 load cases, :674-951)
       DTC_CUDA(cudaMemsetAsync(I.bufs[bP64], 0, vbytes64, s));
       DTC_CUDA(cudaMemsetAsync(I.bufs[bW64], 0, vbytes64, s));
-      apply_k<double, NEN, false, false>(W, dd, I.svox(), fl, X, R64, -1.0, nullptr, nullptr, s, 1);
+      apply_k<double, NEN, false, false>(W, dd, I.svox(), fl, X, R64, -1.0, nullptr, nullptr, s);
       ++L;
       if ((e = run_cg<double, false, NEN>(I, ndom, W, X, R64, B<double>(I, bP64), B<double>(I, bW64), B<double>(I, bDinv64),
                               opt.rtol, nullptr, opt.max_it, L, msg)))
@@ -2669,7 +2336,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
           apply_k<double, NEN, true, false>(W, dd, I.svox(), fl, X, R64, 1.0, nullptr, nullptr, s);
           ++L;
         } else if (nti) {   // first check: X holds the boundary values only, R64 is zero
-          apply_k<double, NEN, false, false>(W, dd, I.svox(), fl, X, R64, -1.0, nullptr, nullptr, s, 1);
+          apply_k<double, NEN, false, false>(W, dd, I.svox(), fl, X, R64, -1.0, nullptr, nullptr, s);
           ++L;
         }
         if (nti) {

@@ -21,11 +21,11 @@
 //
 // One V-cycle per CG iteration, per level l that is not a domain's coarsest:
 //   t_l = omega D_l^-1 b_l                        k_mg_jacobi_flat (fine level: k_blk_update)
-//   r_l = b_l - K_l t_l                           k_mg_matvec<kMgRes>
+//   r_l = b_l - K_l t_l                           k_sweep<kSwRes>
 //   b_{l+1} = P^T r_l                             k_mg_restrict_flat
 //   (level l+1: recurse, or z_{l+1} = K^-1 b)     ...  / k_mg_coarse
 //   t_l += P z_{l+1}                              k_mg_prolong_flat
-//   z_l = t_l + omega D_l^-1 (b_l - K_l t_l)      k_mg_matvec<kMgPost>
+//   z_l = t_l + omega D_l^-1 (b_l - K_l t_l)      k_sweep<kSwPost>
 // Levels >= 2 apply the smoothing step twice before and twice after the coarse correction.
 #pragma once
 
@@ -37,68 +37,6 @@ enum { kMgRes = 0, kMgPost = 1 };
 // node-list entries: (domain << kListShift) | node
 constexpr int kListShift = 40;
 constexpr int64_t kListNodeMask = (int64_t(1) << kListShift) - 1;
-
-// Residual / smoother on one level's interior tiles (the slab sweep of k_matvec).
-//   kMgRes : y = b - K u
-//   kMgPost: y = u + omega D^-1 (b - K u)
-// MINB: CTAs per SM the register allocation is sized for (6: at most 80 registers; 8: 64);
-// xlen: nodes per row of the tile list (kSweepX)
-template <int MODE, int MINB = 6>
-__global__ void __launch_bounds__(kThreads, MINB) k_mg_matvec(const Tile* __restrict__ tiles, const DomDev* __restrict__ doms,
-                                                        const float* __restrict__ svox,
-                                                        const float* __restrict__ binv, const float* __restrict__ b,
-                                                        const float* __restrict__ u, float* __restrict__ y, float omega,
-                                                        const int* __restrict__ dom_active, int xlen) {
-  const Tile t = tiles[blockIdx.x / 3];
-  if (dom_active && !dom_active[t.dom]) return;
-  const DomDev D = doms[t.dom];
-  const int lc = (blockIdx.x % 3) * kLcGroup + (threadIdx.x & 7);
-  const int row = threadIdx.x >> 3;
-  const int yy = t.y0 + (row & 3), zz = t.z0 + (row >> 2);
-  if (yy >= 1 && yy <= D.n[1] - 2 && zz >= 1 && zz <= D.n[2] - 2) {
-    const int sy = D.n[0] * (3 * kNLC), sz = D.n[0] * D.n[1] * (3 * kNLC);
-    const float* rp = u + vec_index(node_index(D, t.x0 - 1, yy, zz), 0, lc);   // plane x0 - 1
-    VoxRow V;
-    float sv[2][2];
-    float cur[3] = {0.f, 0.f, 0.f}, nxt[3] = {0.f, 0.f, 0.f};
-    V.start(svox, D, t.x0 - 1, yy, zz);
-    V.load(sv);
-    bool anyp = (sv[0][0] != 0.f) | (sv[0][1] != 0.f) | (sv[1][0] != 0.f) | (sv[1][1] != 0.f);
-    row_slab<true>(rp, sy, sz, sv, cur, nxt);
-    const int xe = min(D.n[0] - 2, t.x0 + xlen - 1);
-#pragma unroll 1
-    for (int x = t.x0; x <= xe; ++x) {
-      rp += 3 * kNLC;   // plane x
-      ++V.p;
-      V.load(sv);
-      const bool anyc = (sv[0][0] != 0.f) | (sv[0][1] != 0.f) | (sv[1][0] != 0.f) | (sv[1][1] != 0.f);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) { cur[c] = nxt[c]; nxt[c] = 0.f; }
-      row_slab<false>(rp, sy, sz, sv, cur, nxt);
-      if (anyp | anyc) {
-        const int64_t k0 = rp - u;
-        float res[3], bc[3], v[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          bc[c] = b[k0 + c * kNLC];
-          res[c] = bc[c] - (float)(D.scale * (double)cur[c]);
-        }
-        if (MODE == kMgRes) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) v[c] = res[c];
-        } else {
-          float dz[3];
-          block_jacobi(binv, node_index(D, x, yy, zz), omega, res, dz);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) v[c] = __ldg(rp + c * kNLC) + dz[c];
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) y[k0 + c * kNLC] = v[c];
-      }
-      anyp = anyc;
-    }
-  }
-}
 
 // Node-local second half of the residual / smoother when K t was applied by the brick kernel
 // (HEX20 fine level), z holding -K t on entry:

@@ -84,8 +84,7 @@ struct KernelClass {
 
 enum KClassId { kcMatvec32, kcMatvec64, kcUpdate32, kcUpdate64, kcDirection32, kcDirection64, kcColstate,
                 kcReaction, kcProject, kcMgJacobi, kcMgResidual, kcMgPost, kcMgTransfer, kcMgCoarse,
-                kcRotation, kcTuneSimt, kcTuneTc, kcTuneRes4, kcTuneRes5, kcTunePost5, kcTuneApply4, kcTuneApply5,
-                kcTuneF64a, kcTuneF64b, kcGram32, kcHostPack, kcHostMgBuild,
+                kcRotation, kcTuneSimt, kcTuneTc, kcGram32, kcHostPack, kcHostMgBuild,
                 kcNumClasses };   // the last two: host phases (wall ms)
 
 struct SolverStats {
