@@ -831,17 +831,19 @@ struct Work {
   int* err;             // mbarrier time-out flag of the tensor-core kernels
   const Tile *tw = nullptr, *twa = nullptr;   // tiles of the HEX08 sweeps over the interior / all nodes
   int64_t ntw = 0, ntwa = 0;
+  int len = kSweepX;               // their nodes in x
   const Chunk* chunks = nullptr;   // the node list in pieces of one domain (block CG)
   int64_t nchunks = 0;
 };
 
-// One HEX08 sweep over nt tiles.
+// One HEX08 sweep over nt tiles of len nodes in x.
 template <typename T, bool ALL, int MODE>
-void launch_sweep(int64_t nt, cudaStream_t s, const Tile* tiles, const DomDev* dd, const float* svox, const T* u,
-                  T* y, double scale, const float* binv, const T* b, float omega, double* acc, const int* act) {
+void launch_sweep(int64_t nt, int len, cudaStream_t s, const Tile* tiles, const DomDev* dd, const float* svox,
+                  const T* u, T* y, double scale, const float* binv, const T* b, float omega, double* acc,
+                  const int* act) {
   if (nt <= 0) return;
   const unsigned g = (unsigned)(nt * (kNLC / (4 * Lane<T>::kCols)));
-  k_sweep<T, ALL, MODE><<<g, kSweepThreads, kSweepSmem, s>>>(tiles, dd, svox, u, y, scale, binv, b, omega, acc, act);
+  k_sweep<T, ALL, MODE><<<g, kSweepThreads, kSweepSmem, s>>>(tiles, len, dd, svox, u, y, scale, binv, b, omega, acc, act);
 }
 
 template <typename T, bool ALL, int MODE>
@@ -865,8 +867,8 @@ template <typename T, int NEN, bool ALL, bool DOT>
 void apply_k(const Work& W, const DomDev* dd, const float* svox, const uint8_t* fl, const T* u, T* y, double scale,
              double* acc, const int* act, cudaStream_t s) {
   if constexpr (NEN == 8) {
-    launch_sweep<T, ALL, DOT ? kSwApplyDot : kSwApply>(ALL ? W.ntwa : W.ntw, s, ALL ? W.twa : W.tw, dd, svox, u, y,
-                                                       scale, nullptr, nullptr, 0.f, acc, act);
+    launch_sweep<T, ALL, DOT ? kSwApplyDot : kSwApply>(ALL ? W.ntwa : W.ntw, W.len, s, ALL ? W.twa : W.tw, dd, svox,
+                                                       u, y, scale, nullptr, nullptr, 0.f, acc, act);
   } else {
     const T* ke;
     if constexpr (sizeof(T) == 8) ke = W.ke64;
@@ -883,6 +885,20 @@ void apply_k(const Work& W, const DomDev* dd, const float* svox, const uint8_t* 
 
 
 // -------------------------------------------------------------------------------------
+// Sweep tiles of kSweepX nodes in x that a grid of L voxels has at most, and the nodes in x of a list
+// whose domains have so many: a sweep walks its tile plane by plane, so a list that leaves SMs idle (2 CTAs on
+// each of 148, three per tile) is cut shorter -- 4 planes and the one before instead of 16 take a third of the
+// time, for 18 % more work.  One domain of 16^3: fine sweeps 18 - 22 -> 12 - 13 us, its solve 5.2 -> 4.2 ms.
+int64_t sweep_tiles(const int L[3]) {
+  auto up = [](int n, int t) { return (int64_t)((n - 1 + t - 1) / t); };
+  return up(L[0], kSweepX) * up(L[1], kSweepY) * up(L[2], kSweepZ);
+}
+int sweep_length(int64_t tiles) {
+  int len = kSweepX;
+  while (len > 4 && 3 * tiles * (kSweepX / len) < 2 * 148) len /= 2;
+  return len;
+}
+
 // Multigrid hierarchy of one solve (HEX08, FP32 inner solve).  Level 0 is the fine grid
 // already packed; levels >= 1 live in their own node / voxel arrays.  Per level: DomDev for
 // every domain (L = 0 where the domain has no such level), interior tiles of the domains that
@@ -896,6 +912,7 @@ struct MgPlan {
   std::vector<Tile> tiles;
   std::vector<int64_t> sm_off, sm_n, in_off, in_n, all_off, all_n;
   std::vector<int64_t> sw_off, sw_n;                // smoothing tiles of the HEX08 sweeps
+  std::vector<int> sw_len;                          // their nodes in x
   std::vector<int> lists;
   std::vector<int64_t> list_off, list_n;
   std::vector<int64_t> nodes_l;                     // levels >= 1: active interior nodes, (domain << kListShift) | node
@@ -1038,7 +1055,8 @@ constexpr int kMgTwiceFrom = 2;
 // grids are halved as for HEX08.  Every domain's levels are built on their own host thread,
 // then concatenated in domain order (the layout does not depend on the thread count).
 void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<float>& svox0,
-              const std::vector<Tile>& fine_i, const std::vector<Tile>& fine_w, double nu, int nen, int threads) {
+              const std::vector<Tile>& fine_i, const std::vector<Tile>& fine_w, int fine_len, double nu, int nen,
+              int threads) {
   const int ndom = (int)doms0.size();
   double kh[576];
   voxel_stiffness(8, nu, kh);
@@ -1061,6 +1079,21 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
       ++nlev[d];
     }
     nl = std::max(nl, nlev[d]);
+  }
+  // nodes in x of the levels' sweep tiles
+  P.sw_len.assign(nl, fine_len);
+  for (int l = 1; l < nl; ++l) {
+    int64_t tiles = 0;
+    for (int d = 0; d < ndom; ++d) {
+      if (nlev[d] <= l + 1) continue;
+      int n[3];
+      for (int k = 0; k < 3; ++k) {
+        n[k] = doms0[d].L[k];
+        for (int q = doms0[d].m == 2 ? 1 : 0; q < l; ++q) n[k] = (n[k] + 1) / 2;
+      }
+      tiles += sweep_tiles(n);
+    }
+    P.sw_len[l] = sweep_length(tiles);
   }
   // per domain and level >= 1: grid, voxel factors, work lists (offsets filled in later)
   struct Level {
@@ -1129,8 +1162,8 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
       if (nlev[d] > l + 1)
         for (int z0 = 1; z0 <= nz - 2; z0 += kSweepZ)
           for (int y0 = 1; y0 <= ny - 2; y0 += kSweepY)
-            for (int x0 = 1; x0 <= nx - 2; x0 += kSweepX)
-              if (any(x0, y0, z0, 1, nx - 2, ny - 2, nz - 2, kSweepX, kSweepY, kSweepZ))
+            for (int x0 = 1; x0 <= nx - 2; x0 += P.sw_len[l])
+              if (any(x0, y0, z0, 1, nx - 2, ny - 2, nz - 2, P.sw_len[l], kSweepY, kSweepZ))
                 Lv.t_sw.push_back(Tile{d, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
       for (int z = 1; z < nz - 1; ++z)
         for (int y = 1; y < ny - 1; ++y)
@@ -1222,9 +1255,9 @@ struct MgDev {
 
 // The HEX08 residual and post-smoothing sweeps of a level over nt sweep tiles.
 template <int MODE>
-void launch_mg_matvec(int64_t nt, cudaStream_t s, const Tile* t, const DomDev* d, const float* sv, const float* bi,
-                      const float* b, const float* u, float* y, float om, const int* act) {
-  launch_sweep<float, false, MODE == kMgRes ? kSwRes : kSwPost>(nt, s, t, d, sv, u, y, 1.0, bi, b, om, nullptr, act);
+void launch_mg_matvec(int64_t nt, int len, cudaStream_t s, const Tile* t, const DomDev* d, const float* sv,
+                      const float* bi, const float* b, const float* u, float* y, float om, const int* act) {
+  launch_sweep<float, false, MODE == kMgRes ? kSwRes : kSwPost>(nt, len, s, t, d, sv, u, y, 1.0, bi, b, om, nullptr, act);
 }
 
 // t_ready: the fine-level t = omega D^-1 r0 was already written (by k_blk_update)
@@ -1247,7 +1280,7 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   const double mf = I.profile && fine ? I.active_sum(I.dom_mv_flops) : 0;
   const int q0 = fine ? -1 : I.begin(0);
   if (P.list_n[l] > 0) {
-    k_mg_coarse<<<(unsigned)P.list_n[l], 256, 0, s>>>(M.lists + P.list_off[l], dl, M.minv, b, z, act);
+    k_mg_coarse<<<(unsigned)P.list_n[l], kMgCoarseThreads, 0, s>>>(M.lists + P.list_off[l], dl, M.minv, b, z, act);
     ++launches;
   }
   const int64_t nsm = P.sm_n[l];
@@ -1259,6 +1292,7 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   const unsigned g = (unsigned)(3 * nsm);
   const Tile* tsw = M.tiles + P.sw_off[l];        // the sweep tiles
   const int64_t gw = P.sw_n[l];
+  const int sl = P.sw_len[l];
   int q = -1;
   if (!(fine && t_ready)) {
     q = fine ? I.begin(0) : -1;
@@ -1277,7 +1311,7 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   float* cur = t;                  // the smoothed iterate
   float* rbuf = z;                 // the residual handed to the restriction
   if (twice) {
-    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, t, z, om, act);
+    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, t, z, om, act);
     ++launches;
     cur = z;
     rbuf = t;
@@ -1292,9 +1326,9 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   } else if (fine && I.tensor_matvec) {
     launch_sweep_tc(kTcRes, tsm, nsm, dl, sv, fl, bi, b, cur, rbuf, 1.0f, om, nullptr, act, M.err, s);
   } else if (fine) {
-    launch_mg_matvec<kMgRes>(gw, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
+    launch_mg_matvec<kMgRes>(gw, sl, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
   } else {
-    launch_mg_matvec<kMgRes>(gw, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
+    launch_mg_matvec<kMgRes>(gw, sl, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
   }
   if (fine) I.end(kcMgResidual, q, mb + vb, mf);          // t in, r out (mb), b in
   const DomDev* dc = M.doms + (size_t)(l + 1) * M.ndom;
@@ -1329,14 +1363,14 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   } else if (l == 0 && I.tensor_matvec)
     launch_sweep_tc(kTcPost, tsm, nsm, dl, sv, fl, bi, b, t, z, 1.0f, P.omega0, nullptr, act, M.err, s);
   else if (l == 0)
-    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, t, z, P.omega0, act);
+    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega0, act);
   else if (twice) {
     // z holds the corrected iterate: t = z + w D^-1 (b - K z), then z = t + w D^-1 (b - K t)
-    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, z, t, P.omega, act);
-    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
+    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, z, t, P.omega, act);
+    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
     ++launches;
   } else
-    launch_mg_matvec<kMgPost>(gw, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
+    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
   if (fine) I.end(kcMgPost, q, mb + vb + vb / 12, mf);     // t in, z out (mb), b in, D^-1
   if (!fine) I.end(kcMgCoarse, q1, 0, 0);
   launches += 2;
@@ -1580,7 +1614,7 @@ int run_cg_mg(DeviceSolver::Impl& I, int ndom, int nactive, const Work& W, const
   MgPlan Pc;   // offsets and counts of the multigrid lists (no bulk data)
   Pc.nlev = M.P->nlev; Pc.omega = M.P->omega; Pc.omega0 = M.P->omega0;
   Pc.sm_off = M.P->sm_off; Pc.sm_n = M.P->sm_n; Pc.in_off = M.P->in_off; Pc.in_n = M.P->in_n;
-  Pc.sw_off = M.P->sw_off; Pc.sw_n = M.P->sw_n;
+  Pc.sw_off = M.P->sw_off; Pc.sw_n = M.P->sw_n; Pc.sw_len = M.P->sw_len;
   Pc.list_off = M.P->list_off; Pc.list_n = M.P->list_n;
   Pc.nl_off = M.P->nl_off; Pc.nl_n = M.P->nl_n;
   MgDev Mc = M;
@@ -1759,6 +1793,7 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
   const float* b = B<float>(I, bR32);
   const Tile* tsw = M.tiles + M.P->sw_off[0];
   const int64_t gw = M.P->sw_n[0];
+  const int sl = M.P->sw_len[0];
   TuneResult r{0, {0.f, 0.f}};
   int e;
   for (int cand = 0; cand < 2; ++cand) {
@@ -1771,7 +1806,7 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
           launch_ebe_tc(M.bricks0, M.nbricks0, M.doms0, M.svox0, M.flags0, W.ke20tc, M.t0, M.z0, -1.0, nullptr,
                         nullptr, M.err, s);
       } else if (cand == 0) {
-        launch_mg_matvec<kMgPost>(gw, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
+        launch_mg_matvec<kMgPost>(gw, sl, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
       } else {
         launch_sweep_tc(kTcPost, tsm, nsm, M.doms0, M.svox0, M.flags0, M.binv0, b, M.t0, M.z0, 1.0f, M.P->omega0,
                         nullptr, nullptr, M.err, s);
@@ -1792,6 +1827,7 @@ struct HostBatch {
   std::vector<DomDev> doms;
   std::vector<Tile> tiles_i, tiles_a, bricks_i, bricks_a;
   std::vector<Tile> tiles_w, tiles_wa;   // sweep tiles (HEX08) over the interior / all nodes
+  int sweep_len = kSweepX;               // their nodes in x
   std::vector<int64_t> nodes_i;
   std::vector<Chunk> chunks;   // nodes_i cut into pieces of one domain (block CG)
   std::vector<int> nchunk;     // per domain
@@ -1821,14 +1857,18 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
     if (tasks[k].plan->status == DTC_DOMAIN_OK) tidx.push_back((int64_t)k);
   const int ndom_p = (int)tidx.size();
   std::vector<int64_t> vox_offs(ndom_p), node_offs(ndom_p);
-  int64_t vox_total = 0;
+  int64_t vox_total = 0, sweep_total = 0;
   for (int d = 0; d < ndom_p; ++d) {
     const dtc_domain_in& in = *tasks[tidx[d]].in;
     vox_offs[d] = vox_total;
     node_offs[d] = node_total;
     vox_total += in.L[0] * in.L[1] * in.L[2];
+    const int L[3] = {(int)in.L[0], (int)in.L[1], (int)in.L[2]};
+    sweep_total += sweep_tiles(L);
     node_total += (int64_t)(m * in.L[0] + 1) * (m * in.L[1] + 1) * (m * in.L[2] + 1);
   }
+  hb.sweep_len = sweep_length(sweep_total);
+  const int len = hb.sweep_len;
   svox.assign((size_t)vox_total, 0.f);
   // per domain: voxel factors, node activity and work lists (host threads)
   struct Packed {
@@ -1913,13 +1953,13 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
     if (m == 1) {
       for (int z0 = 1; z0 <= nz - 2; z0 += kSweepZ)
         for (int y0 = 1; y0 <= ny - 2; y0 += kSweepY)
-          for (int x0 = 1; x0 <= nx - 2; x0 += kSweepX)
-            if (any_active(x0, y0, z0, kSweepX, kSweepY, kSweepZ, 1, nx - 2, ny - 2, nz - 2))
+          for (int x0 = 1; x0 <= nx - 2; x0 += len)
+            if (any_active(x0, y0, z0, len, kSweepY, kSweepZ, 1, nx - 2, ny - 2, nz - 2))
               out.tw.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
       for (int z0 = 0; z0 <= nz - 1; z0 += kSweepZ)
         for (int y0 = 0; y0 <= ny - 1; y0 += kSweepY)
-          for (int x0 = 0; x0 <= nx - 1; x0 += kSweepX)
-            if (any_active(x0, y0, z0, kSweepX, kSweepY, kSweepZ, 0, nx - 1, ny - 1, nz - 1))
+          for (int x0 = 0; x0 <= nx - 1; x0 += len)
+            if (any_active(x0, y0, z0, len, kSweepY, kSweepZ, 0, nx - 1, ny - 1, nz - 1))
               out.twa.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
     }
     for (int z0 = 0; z0 <= nz - 1; z0 += kTileZ)
@@ -1967,7 +2007,7 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
   // multigrid plan of the mixed inner solve (HEX08 levels; HEX20 starts with p-coarsening)
   if (opt.precision == DTC_PREC_MIXED && opt.inner_precond == 2 && !tiles_i.empty()) {
     const auto tb = std::chrono::steady_clock::now();
-    build_mg(hb.mg, doms, svox, tiles_i, hb.tiles_w, nu, NEN, opt.host_threads);
+    build_mg(hb.mg, doms, svox, tiles_i, hb.tiles_w, hb.sweep_len, nu, NEN, opt.host_threads);
     hb.has_mg = true;
     hb.ms_mg = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tb).count();
   }
@@ -2151,6 +2191,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   W.ntw = ntw;
   W.twa = B<Tile>(I, bTilesWa);
   W.ntwa = ntwa;
+  W.len = hb.sweep_len;
   const DomDev* dd = B<DomDev>(I, bDoms);
   uint8_t* fl = B<uint8_t>(I, bFlags);
   double* X = B<double>(I, bX);
@@ -2174,7 +2215,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
       mgp = std::move(hb.mg);
     } else {
       const auto tb = std::chrono::steady_clock::now();
-      build_mg(mgp, doms, svox, tiles_i, hb.tiles_w, nu, NEN, opt.host_threads);
+      build_mg(mgp, doms, svox, tiles_i, hb.tiles_w, hb.sweep_len, nu, NEN, opt.host_threads);
       stats_.kc[kcHostMgBuild].ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tb).count();
       stats_.kc[kcHostMgBuild].launches += 1;
     }

@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(256) k_mg_prolong_flat(const int64_t* __restri
   }
 }
 
-// b_c = P^T r_f (full weighting) over a coarse level's node list.
+// b_c = P^T r_f (full weighting) over a coarse level's node list.  Branch-free, so that the loads of a z plane
+// are in flight together (coarse levels of 24 domains of 32^3: 21 -> 16 us).
 __global__ void __launch_bounds__(256) k_mg_restrict_flat(const int64_t* __restrict__ list, int64_t nitems,
                                                           const DomDev* __restrict__ doms_c,
                                                           const DomDev* __restrict__ doms_f,
@@ -165,18 +166,22 @@ __global__ void __launch_bounds__(256) k_mg_restrict_flat(const int64_t* __restr
   float4 s[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) s[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+  // the 27 fine nodes; one past the grid's far side (odd voxel count) has weight 0, its neighbour's address
+#pragma unroll 1
   for (int dz = -1; dz <= 1; ++dz) {
     const int fz = 2 * z + dz;
-    if (fz > F.n[2] - 1) continue;
+    const float wz = fz > F.n[2] - 1 ? 0.f : dz ? 0.5f : 1.f;
+    const int64_t pz = node_index(F, 0, 0, min(fz, F.n[2] - 1));
+#pragma unroll
     for (int dy = -1; dy <= 1; ++dy) {
       const int fy = 2 * y + dy;
-      if (fy > F.n[1] - 1) continue;
+      const float wy = fy > F.n[1] - 1 ? 0.f : dy ? 0.5f * wz : wz;
+      const int64_t py = pz + (int64_t)F.n[0] * min(fy, F.n[1] - 1);
 #pragma unroll
       for (int dx = -1; dx <= 1; ++dx) {
         const int fx = 2 * x + dx;
-        if (fx > F.n[0] - 1) continue;
-        const float wgt = (dx ? 0.5f : 1.f) * (dy ? 0.5f : 1.f) * (dz ? 0.5f : 1.f);
-        const int64_t k = vec_index(node_index(F, fx, fy, fz), 0, lc0);
+        const float wgt = fx > F.n[0] - 1 ? 0.f : dx ? 0.5f * wy : wy;
+        const int64_t k = vec_index(py + min(fx, F.n[0] - 1), 0, lc0);
 #pragma unroll
         for (int c = 0; c < 3; ++c) fmaq(wgt, ldq(r_f + k + c * kNLC), s[c]);
       }
@@ -225,16 +230,21 @@ __global__ void __launch_bounds__(256) k_mg_jacobi_flat(const int64_t* __restric
 }
 
 // Coarsest level: z = Minv b over the <= 27 interior nodes of each listed domain (one CTA per
-// domain, Minv 81 x 81 row-major on the DOFs 3 * ((x-1) + 3 (y-1) + 9 (z-1)) + c).
-__global__ void __launch_bounds__(256) k_mg_coarse(const int* __restrict__ list, const DomDev* __restrict__ doms,
-                                                   const float* __restrict__ minv, const float* __restrict__ b,
-                                                   float* __restrict__ z, const int* __restrict__ dom_active) {
-  __shared__ float sb[kMgDenseN * kNLC];
+// domain, Minv 81 x 81 symmetric on the DOFs 3 * ((x-1) + 3 (y-1) + 9 (z-1)) + c).  A thread owns one DOF and
+// 8 load cases; the symmetric matrix is read by columns, so that a warp reads consecutive entries.  Bound by
+// the latency of its 81 steps: 36 -> 21 us (24 domains; one thread per output read a row of the matrix).
+constexpr int kMgCoarseThreads = 3 * 96;
+__global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarse(const int* __restrict__ list,
+                                                                const DomDev* __restrict__ doms,
+                                                                const float* __restrict__ minv,
+                                                                const float* __restrict__ b, float* __restrict__ z,
+                                                                const int* __restrict__ dom_active) {
+  __shared__ __align__(16) float sb[kMgDenseN * kNLC];
   const int d = list[blockIdx.x];
   if (dom_active && !dom_active[d]) return;
   const DomDev D = doms[d];
   const int ix = D.n[0] - 2, iy = D.n[1] - 2, iz = D.n[2] - 2;   // interior nodes per axis (<= 3)
-  for (int i = threadIdx.x; i < kMgDenseN * kNLC; i += blockDim.x) {
+  for (int i = threadIdx.x; i < kMgDenseN * kNLC; i += kMgCoarseThreads) {
     const int lc = i % kNLC, dof = i / kNLC, node = dof / 3, c = dof % 3;
     const int x = node % 3, y = (node / 3) % 3, zc = node / 9;
     float v = 0.f;
@@ -242,15 +252,24 @@ __global__ void __launch_bounds__(256) k_mg_coarse(const int* __restrict__ list,
     sb[i] = v;
   }
   __syncthreads();
-  const float* M = minv + (int64_t)d * kMgDenseN * kMgDenseN;
-  for (int i = threadIdx.x; i < kMgDenseN * kNLC; i += blockDim.x) {
-    const int lc = i % kNLC, dof = i / kNLC, node = dof / 3, c = dof % 3;
-    const int x = node % 3, y = (node / 3) % 3, zc = node / 9;
-    if (x >= ix || y >= iy || zc >= iz) continue;
-    float s = 0.f;
-    for (int k = 0; k < kMgDenseN; ++k) s = fmaf(__ldg(M + dof * kMgDenseN + k), sb[k * kNLC + lc], s);
-    z[vec_index(node_index(D, x + 1, y + 1, zc + 1), c, lc)] = s;
+  const int dof = threadIdx.x % 96, lc0 = 8 * (threadIdx.x / 96);
+  const int node = dof / 3, c = dof % 3, x = node % 3, y = (node / 3) % 3, zc = node / 9;
+  if (dof >= kMgDenseN || x >= ix || y >= iy || zc >= iz) return;
+  const float* M = minv + (int64_t)d * kMgDenseN * kMgDenseN + dof;
+  float s[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) s[q] = 0.f;
+#pragma unroll 9
+  for (int k = 0; k < kMgDenseN; ++k) {
+    const float m = __ldg(M + k * kMgDenseN);
+    const float4 v0 = *reinterpret_cast<const float4*>(sb + k * kNLC + lc0);
+    const float4 v1 = *reinterpret_cast<const float4*>(sb + k * kNLC + lc0 + 4);
+    s[0] = fmaf(m, v0.x, s[0]); s[1] = fmaf(m, v0.y, s[1]); s[2] = fmaf(m, v0.z, s[2]); s[3] = fmaf(m, v0.w, s[3]);
+    s[4] = fmaf(m, v1.x, s[4]); s[5] = fmaf(m, v1.y, s[5]); s[6] = fmaf(m, v1.z, s[6]); s[7] = fmaf(m, v1.w, s[7]);
   }
+  float* zp = z + vec_index(node_index(D, x + 1, y + 1, zc + 1), c, lc0);
+  *reinterpret_cast<float4*>(zp) = make_float4(s[0], s[1], s[2], s[3]);
+  *reinterpret_cast<float4*>(zp + 4) = make_float4(s[4], s[5], s[6], s[7]);
 }
 
 }  // namespace dtc

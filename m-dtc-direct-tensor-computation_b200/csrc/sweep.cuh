@@ -211,7 +211,7 @@ static_assert(kSweepY == 8 && kSweepZ % 2 == 0, "the dealing of rows to threads"
 
 enum { kSwApply = 0, kSwApplyDot = 1, kSwRes = 2, kSwPost = 3 };
 
-// On the node rows of the listed tiles (interior nodes; ALL: every node of the grid):
+// On the node rows of the listed tiles, len <= kSweepX nodes in x (interior nodes; ALL: every node of the grid):
 //   kSwApply: y = scale K u;  kSwApplyDot: acc[dom][load case] += u . y as well
 //   kSwRes  : y = b - K u
 //   kSwPost : y = u + omega D^-1 (b - K u)
@@ -225,7 +225,7 @@ enum { kSwApply = 0, kSwApplyDot = 1, kSwRes = 2, kSwPost = 3 };
 // 361 -> 249 us, post-smoothing 375 -> 298, CG application 319 -> 224; FP64 application, 27 x 20^3,
 // 116 -> 85.  Loading the planes into registers one step ahead took 278, 331 and 255 us.
 template <typename T, bool ALL, int MODE>
-__global__ void __launch_bounds__(kSweepThreads, 2) k_sweep(const Tile* __restrict__ tiles,
+__global__ void __launch_bounds__(kSweepThreads, 2) k_sweep(const Tile* __restrict__ tiles, int len,
                                                             const DomDev* __restrict__ doms,
                                                             const float* __restrict__ svox,
                                                             const T* __restrict__ u, T* __restrict__ y,
@@ -253,14 +253,14 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_sweep(const Tile* __restri
   const int lc0 = (blockIdx.x % kGroups) * (4 * L::kCols), lc = lc0 + (tid & 3) * L::kCols;
   const int vy = t.y0 - 1 + j, vz = t.z0 - 1 + k;   // voxel row; node row (vy, vz) is finished here
   const int hi = ALL ? 1 : 2;
-  const int xe = min(D.n[0] - hi, t.x0 + kSweepX - 1);
+  const int xe = min(D.n[0] - hi, t.x0 + len - 1);
   if (tid == 0) kept_any = 0;
   for (int e = tid; e < kVoxRows * kStep; e += kSweepThreads) {
     const int q = e / kStep, i = e % kStep;
     int jq, kq;
     slot_row(q, jq, kq);
     const int x = t.x0 - 1 + i, yy = t.y0 - 1 + jq, zz = t.z0 - 1 + kq;
-    const bool in = x >= 0 && yy >= 0 && zz >= 0 && x < D.L[0] && yy < D.L[1] && zz < D.L[2];
+    const bool in = i <= len && x >= 0 && yy >= 0 && zz >= 0 && x < D.L[0] && yy < D.L[1] && zz < D.L[2];
     const int64_t at = in ? x + (int64_t)D.L[0] * (yy + (int64_t)D.L[1] * zz) : 0;
     const float s = __ldg(svox + D.vox_off + at);
     fac[e] = in ? s : 0.f;
