@@ -5,16 +5,18 @@
 // off-diagonal energy of B^T E B (CR1: rows 1-4 x cols 5-6; CR2: all 12 upper off-diagonal
 // entries), takes the first minimum in column-major order (MINLOC), then refines in a
 // +-1 step window at 10x finer resolution until the minimum changes by < 1e-9 or 16 rounds.
-// Here one thread evaluates one candidate; a block argmin keeps MINLOC's tie rule (smallest
-// linear index, alpha fastest).  This file is compiled with --fmad=false so every
+// Here one thread evaluates the candidates about one axis; the argmin reductions keep MINLOC's tie rule
+// (smallest linear index, alpha fastest).  This file is compiled with --fmad=false so every
 // criterion is evaluated with the same rounding steps as the written expression.
 //
 // Sines and cosines: the 1-degree sweep reads two tables built on the host, each refinement
 // level builds its 3 x 21 values in shared memory; all of them are the correctly rounded
 // values (ddmath.h), the same on the host and the device, so the argmin indices do not
 // depend on which math library evaluated them.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -26,6 +28,8 @@
 #include "kernels.cuh"
 #include "solver.h"
 
+namespace cg = cooperative_groups;
+
 namespace dtc {
 
 __constant__ double c_cosd[181], c_sind[181];
@@ -33,62 +37,121 @@ __constant__ double c_cosd[181], c_sind[181];
 namespace {
 
 constexpr int kSweepA = 181, kSweepP = 181, kSweepE = 91;
-constexpr int64_t kSweepN = (int64_t)kSweepA * kSweepP * kSweepE;
-constexpr int kSweepBlocks = 64;
-constexpr int kRotThreads = 256;
+constexpr int kAxes = kSweepP * kSweepE;
+constexpr int kSegments = 8;            // the sweep's work item: one axis, an eighth of the angles about it
+constexpr int kSegLen = (kSweepA + kSegments - 1) / kSegments;
+constexpr int kSweepBlocks = 64;        // per tensor, when there are many
+constexpr int kSweepFill = 888;         // CTAs that fill the card twice (3 on each of 148 SMs)
+constexpr int kSweepThreadsRot = 128;
+// refinement of one (tensor, criterion): a cluster of 7 CTAs, an item is one of 21 x 21 axes and a part of the angles
+constexpr int kRefineCtas = 7, kRefineAxes = 21 * 21 / kRefineCtas, kRefineThreads = 64;   // per part
+static_assert(kRefineAxes * kRefineCtas == 21 * 21 && kRefineAxes <= kRefineThreads, "an item per thread");
 
-__device__ __forceinline__ void criteria(const double* E, double ca, double sa, double cp, double sp, double ce,
-                                         double se, double& c1, double& c2) {
-  double n0 = cp * se, n1 = sp * se, n2 = ce;
-  const double nr = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
-  n0 = n0 / nr; n1 = n1 / nr; n2 = n2 / nr;
+// The axis of a candidate rotation and the products of its components.
+struct Axis {
+  double n0, n1, n2, n00, n11, n22, n12, n13, n23;
+  __device__ __forceinline__ Axis(double cp, double sp, double ce, double se) {
+    n0 = cp * se; n1 = sp * se; n2 = ce;
+    const double nr = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
+    n0 = n0 / nr; n1 = n1 / nr; n2 = n2 / nr;
+    n00 = n0 * n0; n11 = n1 * n1; n22 = n2 * n2;
+    n12 = n0 * n1; n13 = n0 * n2; n23 = n1 * n2;
+  }
+};
+
+// Criteria of the rotation by (ca, sa) about an axis (WHICH bit 0: CR1, bit 1: CR2), every expression in the
+// reference's order.  Both criteria contain the squares of t15, t25, t35 and t45, and CR2 all terms of CR1:
+// once such a sum alone is above what some candidate is known to reach (most1, most2: with a margin far above
+// the rounding of a dozen terms), the candidate cannot be the first minimum, and the criterion is returned as
+// infinity.  Of rotated orthotropic tensors with noise 46 to 89 of 100 candidates end before the
+// second column of the product and 2 to 12 reach the last.
+template <int WHICH>
+__device__ __forceinline__ void criteria(const volatile double* E, const Axis& x, double ca, double sa, double most1,
+                                         double most2, double& c1, double& c2) {
   const double omc = 1.0 - ca;
-  const double n12 = n0 * n1, n13 = n0 * n2, n23 = n1 * n2;
-  const double a11 = ca + n0 * n0 * omc, a22 = ca + n1 * n1 * omc, a33 = ca + n2 * n2 * omc;
-  const double a12 = n12 * omc - n2 * sa, a21 = n12 * omc + n2 * sa;
-  const double a13 = n13 * omc + n1 * sa, a31 = n13 * omc - n1 * sa;
-  const double a23 = n23 * omc - n0 * sa, a32 = n23 * omc + n0 * sa;
+  double a11 = ca + x.n00 * omc, a22 = ca + x.n11 * omc, a33 = ca + x.n22 * omc;
+  double a12 = x.n12 * omc - x.n2 * sa, a21 = x.n12 * omc + x.n2 * sa;
+  double a13 = x.n13 * omc + x.n1 * sa, a31 = x.n13 * omc - x.n1 * sa;
+  double a23 = x.n23 * omc - x.n0 * sa, a32 = x.n23 * omc + x.n0 * sa;
+  // the columns of B are formed again for each column j of the product instead of kept: 72 registers less
+  auto again = [&]() {
+    asm volatile("" : "+d"(a11), "+d"(a12), "+d"(a13), "+d"(a21), "+d"(a22), "+d"(a23), "+d"(a31), "+d"(a32),
+                      "+d"(a33)::"memory");
+  };
   const double s2 = 1.4142135623730951;  // sqrt(2), the value std::sqrt(2.0) rounds to
-  double Bm[6][7];  // Bm[r][c] = B(r+1, c), c = 1..6
-  Bm[0][1] = a11 * a11; Bm[1][1] = a21 * a21; Bm[2][1] = a31 * a31;
-  Bm[3][1] = s2 * a21 * a11; Bm[4][1] = s2 * a11 * a31; Bm[5][1] = s2 * a21 * a31;
-  Bm[0][2] = a12 * a12; Bm[1][2] = a22 * a22; Bm[2][2] = a32 * a32;
-  Bm[3][2] = s2 * a22 * a12; Bm[4][2] = s2 * a12 * a32; Bm[5][2] = s2 * a22 * a32;
-  Bm[0][3] = a13 * a13; Bm[1][3] = a23 * a23; Bm[2][3] = a33 * a33;
-  Bm[3][3] = s2 * a23 * a13; Bm[4][3] = s2 * a13 * a33; Bm[5][3] = s2 * a23 * a33;
-  Bm[0][4] = s2 * a11 * a12; Bm[1][4] = s2 * a21 * a22; Bm[2][4] = s2 * a31 * a32;
-  Bm[3][4] = a21 * a12 + a22 * a11; Bm[4][4] = a11 * a32 + a12 * a31; Bm[5][4] = a21 * a32 + a22 * a31;
-  Bm[0][5] = s2 * a11 * a13; Bm[1][5] = s2 * a21 * a23; Bm[2][5] = s2 * a31 * a33;
-  Bm[3][5] = a21 * a13 + a23 * a11; Bm[4][5] = a11 * a33 + a13 * a31; Bm[5][5] = a21 * a33 + a23 * a31;
-  Bm[0][6] = s2 * a12 * a13; Bm[1][6] = s2 * a22 * a23; Bm[2][6] = s2 * a32 * a33;
-  Bm[3][6] = a22 * a13 + a23 * a12; Bm[4][6] = a12 * a33 + a13 * a32; Bm[5][6] = a22 * a33 + a23 * a32;
+  auto square = [&](double p, double q, double r, double (&B)[6]) {   // columns 1 to 3 from (p, q, r)
+    B[0] = p * p; B[1] = q * q; B[2] = r * r;
+    B[3] = s2 * q * p; B[4] = s2 * p * r; B[5] = s2 * q * r;
+  };
+  auto mixed = [&](double p1, double q1, double r1, double p2, double q2, double r2, double (&B)[6]) {   // 4 to 6
+    B[0] = s2 * p1 * p2; B[1] = s2 * q1 * q2; B[2] = s2 * r1 * r2;
+    B[3] = q1 * p2 + q2 * p1; B[4] = p1 * r2 + p2 * r1; B[5] = q1 * r2 + q2 * r1;
+  };
   // S_j(r) = sum_{c=6..1} B(c,j) E(r,c), then T(i,j) = sum_{r=6..1} B(r,i) S_j(r)
-  double S[3][6];
-#pragma unroll
-  for (int jj = 0; jj < 3; ++jj) {
-    const int j = 4 + jj;
+  double S[6];
+  auto column = [&](const double (&B)[6]) {
 #pragma unroll
     for (int r = 0; r < 6; ++r) {
-      double s = Bm[5][j] * E[r + 6 * 5];
+      double s = B[5] * E[r + 6 * 5];
 #pragma unroll
-      for (int c = 4; c >= 0; --c) s = s + Bm[c][j] * E[r + 6 * c];
-      S[jj][r] = s;
+      for (int c = 4; c >= 0; --c) s = s + B[c] * E[r + 6 * c];
+      S[r] = s;
     }
-  }
-  auto T = [&](int i, int j) {
-    const double* Sj = S[j - 4];
-    double t = Bm[5][i] * Sj[5];
+  };
+  auto T = [&](const double (&B)[6]) {
+    double t = B[5] * S[5];
 #pragma unroll
-    for (int r = 4; r >= 0; --r) t = t + Bm[r][i] * Sj[r];
+    for (int r = 4; r >= 0; --r) t = t + B[r] * S[r];
     return t;
   };
-  const double t14 = T(1, 4), t15 = T(1, 5), t16 = T(1, 6), t24 = T(2, 4), t25 = T(2, 5), t26 = T(2, 6);
-  const double t34 = T(3, 4), t35 = T(3, 5), t36 = T(3, 6), t45 = T(4, 5), t46 = T(4, 6), t56 = T(5, 6);
-  c1 = t15 * t15 + t16 * t16 + t25 * t25 + t26 * t26 + t35 * t35 + t36 * t36 + t45 * t45 + t46 * t46;
-  c2 = t14 * t14 + t15 * t15 + t16 * t16 + t24 * t24 + t25 * t25 + t26 * t26 + t34 * t34 + t35 * t35 + t36 * t36 +
-       t45 * t45 + t46 * t46 + t56 * t56;
-  if (!(c1 == c1)) c1 = INFINITY;
-  if (!(c2 == c2)) c2 = INFINITY;
+  c1 = c2 = INFINITY;
+  const double most = fmax(most1, most2);
+  double B[6];
+  mixed(a11, a21, a31, a13, a23, a33, B);
+  column(B);
+  square(a11, a21, a31, B);
+  const double t15 = T(B);
+  square(a12, a22, a32, B);
+  const double t25 = T(B);
+  if (t15 * t15 + t25 * t25 > most) return;
+  square(a13, a23, a33, B);
+  const double t35 = T(B);
+  mixed(a11, a21, a31, a12, a22, a32, B);
+  const double t45 = T(B);
+  const double part5 = t15 * t15 + t25 * t25 + t35 * t35 + t45 * t45;
+  if (part5 > most) return;
+  again();
+  mixed(a12, a22, a32, a13, a23, a33, B);
+  column(B);
+  square(a11, a21, a31, B);
+  const double t16 = T(B);
+  square(a12, a22, a32, B);
+  const double t26 = T(B);
+  if (part5 + (t16 * t16 + t26 * t26) > most) return;
+  square(a13, a23, a33, B);
+  const double t36 = T(B);
+  mixed(a11, a21, a31, a12, a22, a32, B);
+  const double t46 = T(B);
+  if (WHICH & 1) {
+    c1 = t15 * t15 + t16 * t16 + t25 * t25 + t26 * t26 + t35 * t35 + t36 * t36 + t45 * t45 + t46 * t46;
+    if (!(c1 == c1)) c1 = INFINITY;
+  }
+  if ((WHICH & 2) && !(part5 + (t16 * t16 + t26 * t26 + t36 * t36 + t46 * t46) > most2)) {
+    again();
+    mixed(a11, a21, a31, a13, a23, a33, B);
+    const double t56 = T(B);
+    mixed(a11, a21, a31, a12, a22, a32, B);
+    column(B);
+    square(a11, a21, a31, B);
+    const double t14 = T(B);
+    square(a12, a22, a32, B);
+    const double t24 = T(B);
+    square(a13, a23, a33, B);
+    const double t34 = T(B);
+    c2 = t14 * t14 + t15 * t15 + t16 * t16 + t24 * t24 + t25 * t25 + t26 * t26 + t34 * t34 + t35 * t35 + t36 * t36 +
+         t45 * t45 + t46 * t46 + t56 * t56;
+    if (!(c2 == c2)) c2 = INFINITY;
+  }
 }
 
 struct ArgMin {
@@ -99,57 +162,104 @@ __device__ __forceinline__ bool better(const ArgMin& a, const ArgMin& b) {
   return a.v < b.v || (a.v == b.v && a.i < b.i);
 }
 
-__device__ ArgMin block_argmin(ArgMin m, ArgMin* sh) {
-  sh[threadIdx.x] = m;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w && better(sh[threadIdx.x + w], sh[threadIdx.x])) sh[threadIdx.x] = sh[threadIdx.x + w];
-    __syncthreads();
+// The best of all threads of the CTA, in every thread.
+__device__ __forceinline__ ArgMin block_argmin(ArgMin m, ArgMin* sh) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    ArgMin q;
+    q.v = __shfl_xor_sync(0xffffffffu, m.v, o);
+    q.i = __shfl_xor_sync(0xffffffffu, m.i, o);
+    if (better(q, m)) m = q;
   }
-  ArgMin r = sh[0];
   __syncthreads();
-  return r;
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+  __syncthreads();
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
+    if (better(sh[w], m)) m = sh[w];
+  return m;
 }
 
-__global__ void __launch_bounds__(kRotThreads) k_rot_sweep(const double* __restrict__ ee, ArgMin* __restrict__ part) {
+// 1-degree sweep: a thread evaluates the angles of one segment about one axis, whose normalisation (a square
+// root and three divisions) it does once.  The CTA first evaluates a coarse subset of the same grid: the
+// smallest values there bound what a candidate may reach, and the bounds shrink as its threads find better ones.
+// Bound by the FP64 pipe (80 % busy at 12 warps an SM; the register file holds no more): 66 us a tensor when there
+// are many, 4.00 ms for 64; one CTA row of angles per thread without the bounds took 6.32.  A single tensor is
+// spread over every SM twice over: 0.10 ms, 0.24 with 64 CTAs.
+__global__ void __launch_bounds__(kSweepThreadsRot, 3) k_rot_sweep(const double* __restrict__ ee,
+                                                                ArgMin* __restrict__ part) {
   __shared__ double E[36];
-  __shared__ ArgMin sh[kRotThreads];
+  __shared__ ArgMin sh[kSweepThreadsRot / 32];
   const int dom = blockIdx.y;
   if (threadIdx.x < 36) E[threadIdx.x] = ee[(int64_t)dom * 36 + threadIdx.x];
   __syncthreads();
+  __shared__ long long most[2];   // bits of the bounds, which are not negative: their order is that of the numbers
+  {
+    ArgMin b1{INFINITY, INT64_MAX}, b2{INFINITY, INT64_MAX};
+    if (threadIdx.x < 6 * 6 * 3) {
+      const int ia = 30 * (threadIdx.x % 6), ip = 30 * (threadIdx.x / 6 % 6), ie = 45 * (threadIdx.x / 36);
+      criteria<3>(E, Axis(c_cosd[ip], c_sind[ip], c_cosd[ie], c_sind[ie]), c_cosd[ia], c_sind[ia], INFINITY,
+                  INFINITY, b1.v, b2.v);
+    }
+    b1 = block_argmin(b1, sh);
+    b2 = block_argmin(b2, sh);
+    if (threadIdx.x == 0) {
+      most[0] = __double_as_longlong(b1.v * (1.0 + 1e-9));
+      most[1] = __double_as_longlong(b2.v * (1.0 + 1e-9));
+    }
+    __syncthreads();
+  }
   ArgMin b1{INFINITY, INT64_MAX}, b2{INFINITY, INT64_MAX};
-  for (int64_t idx = (int64_t)blockIdx.x * kRotThreads + threadIdx.x; idx < kSweepN;
-       idx += (int64_t)gridDim.x * kRotThreads) {
-    const int ia = (int)(idx % kSweepA), ip = (int)((idx / kSweepA) % kSweepP), ie = (int)(idx / (kSweepA * kSweepP));
-    double c1, c2;
-    criteria(E, c_cosd[ia], c_sind[ia], c_cosd[ip], c_sind[ip], c_cosd[ie], c_sind[ie], c1, c2);
-    if (c1 < b1.v) { b1.v = c1; b1.i = idx; }
-    if (c2 < b2.v) { b2.v = c2; b2.i = idx; }
+  for (int item = blockIdx.x * kSweepThreadsRot + threadIdx.x; item < kAxes * kSegments;
+       item += gridDim.x * kSweepThreadsRot) {
+    const int axis = item % kAxes, a0 = item / kAxes * kSegLen, a1 = min(a0 + kSegLen, kSweepA);
+    const int ip = axis % kSweepP, ie = axis / kSweepP;
+    const Axis x(c_cosd[ip], c_sind[ip], c_cosd[ie], c_sind[ie]);
+    const double most1 = __longlong_as_double(*(volatile long long*)&most[0]);
+    const double most2 = __longlong_as_double(*(volatile long long*)&most[1]);
+    for (int ia = a0; ia < a1; ++ia) {
+      double c1, c2;
+      criteria<3>(E, x, c_cosd[ia], c_sind[ia], most1, most2, c1, c2);
+      const int64_t idx = ia + (int64_t)kSweepA * axis;
+      // a thread's items do not come in index order: ties go to the smaller index
+      if (c1 < b1.v || (c1 == b1.v && idx < b1.i && c1 < INFINITY)) { b1.v = c1; b1.i = idx; }
+      if (c2 < b2.v || (c2 == b2.v && idx < b2.i && c2 < INFINITY)) { b2.v = c2; b2.i = idx; }
+    }
+    const double own1 = b1.v * (1.0 + 1e-9), own2 = b2.v * (1.0 + 1e-9);
+    if (own1 < most1) atomicMin(&most[0], __double_as_longlong(own1));
+    if (own2 < most2) atomicMin(&most[1], __double_as_longlong(own2));
   }
   const ArgMin r1 = block_argmin(b1, sh);
   const ArgMin r2 = block_argmin(b2, sh);
   if (threadIdx.x == 0) {
-    part[((int64_t)dom * kSweepBlocks + blockIdx.x) * 2 + 0] = r1;
-    part[((int64_t)dom * kSweepBlocks + blockIdx.x) * 2 + 1] = r2;
+    part[((int64_t)dom * gridDim.x + blockIdx.x) * 2 + 0] = r1;
+    part[((int64_t)dom * gridDim.x + blockIdx.x) * 2 + 1] = r2;
   }
 }
 
-// One block per (domain, criterion): reduce the sweep, then the x10 refinement loop.
-__global__ void __launch_bounds__(kRotThreads) k_rot_refine(const double* __restrict__ ee,
-                                                            const ArgMin* __restrict__ part, double pi_div_180,
-                                                            int64_t* __restrict__ ang_out, int* __restrict__ jj_out,
-                                                            double* __restrict__ crit_out) {
+// CTAs per tensor of the sweep: enough to fill the card, at least kSweepBlocks.
+int sweep_blocks(int64_t n) { return (int)std::max<int64_t>(kSweepBlocks, kSweepFill / std::max<int64_t>(n, 1)); }
+
+// One cluster per (domain, criterion): reduce the sweep, then the x10 refinement loop, the best of a level
+// exchanged through the cluster's shared memories.  Bound by the serial chain of a level: its sines and cosines, 11 or 21
+// candidates one after the other, the reduction.  One tensor 0.28 ms, 0.51 with one CTA per search; 64 tensors
+// 0.77 ms (0.79).
+template <int PARTS>
+__global__ void __cluster_dims__(kRefineCtas, 1, 1) __launch_bounds__(kRefineThreads * PARTS, 6 / PARTS)
+    k_rot_refine(const double* __restrict__ ee, const ArgMin* __restrict__ part, int nblocks, double pi_div_180,
+                 int64_t* __restrict__ ang_out, int* __restrict__ jj_out, double* __restrict__ crit_out) {
   __shared__ double E[36];
-  __shared__ ArgMin sh[kRotThreads];
+  __shared__ ArgMin sh[kRefineThreads * PARTS / 32];
+  __shared__ ArgMin level_best[2];   // of this CTA; written for alternate levels
   __shared__ double tsin[3][21], tcos[3][21];
-  const int dom = blockIdx.x, which = blockIdx.y;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int dom = blockIdx.x / kRefineCtas, rank = (int)cluster.block_rank();
+  const int which = 1 - (int)blockIdx.y;   // CR2, the longer one, first
   if (threadIdx.x < 36) E[threadIdx.x] = ee[(int64_t)dom * 36 + threadIdx.x];
   ArgMin m{INFINITY, INT64_MAX};
-  for (int b = threadIdx.x; b < kSweepBlocks; b += kRotThreads) {
-    const ArgMin q = part[((int64_t)dom * kSweepBlocks + b) * 2 + which];
+  for (int b = threadIdx.x; b < nblocks; b += kRefineThreads * PARTS) {
+    const ArgMin q = part[((int64_t)dom * nblocks + b) * 2 + which];
     if (better(q, m)) m = q;
   }
-  __syncthreads();
   const ArgMin s0 = block_argmin(m, sh);
   int64_t a[3];
   if (s0.i == INT64_MAX) { a[0] = a[1] = a[2] = 0; }
@@ -157,7 +267,10 @@ __global__ void __launch_bounds__(kRotThreads) k_rot_refine(const double* __rest
   double prev = s0.v, cur = s0.v;
   double div = pi_div_180;
   int jj = 1;
-  for (;;) {
+  const int slot = (int)threadIdx.x % kRefineThreads, part_of = (int)threadIdx.x / kRefineThreads;
+  const int axis = rank * kRefineAxes + slot;
+  constexpr int kEach = (21 + PARTS - 1) / PARTS;
+  for (;;) {   // every CTA of the cluster takes the same decisions
     const int64_t lo[3] = {(a[0] - 1) * 10, (a[1] - 1) * 10, (a[2] - 1) * 10};
     div = div * 0.1;
     if (threadIdx.x < 63) {
@@ -169,26 +282,50 @@ __global__ void __launch_bounds__(kRotThreads) k_rot_refine(const double* __rest
     }
     __syncthreads();
     ArgMin w{INFINITY, INT64_MAX};
-    for (int t = threadIdx.x; t < 21 * 21 * 21; t += kRotThreads) {
-      const int i0 = t % 21, i1 = (t / 21) % 21, i2 = t / 441;
-      double c1, c2;
-      criteria(E, tcos[0][i0], tsin[0][i0], tcos[1][i1], tsin[1][i1], tcos[2][i2], tsin[2][i2], c1, c2);
-      const double c = which == 0 ? c1 : c2;
-      if (c < w.v) { w.v = c; w.i = t; }
+    if (slot < kRefineAxes) {
+      const int i1 = axis % 21, i2 = axis / 21;
+      const Axis x(tcos[1][i1], tsin[1][i1], tcos[2][i2], tsin[2][i2]);
+      for (int i0 = kEach * part_of; i0 < min(kEach * part_of + kEach, 21); ++i0) {
+        double c1, c2;
+        const double most = w.v * (1.0 + 1e-9);
+        if (which == 0) criteria<1>(E, x, tcos[0][i0], tsin[0][i0], most, -INFINITY, c1, c2);
+        else criteria<2>(E, x, tcos[0][i0], tsin[0][i0], -INFINITY, most, c1, c2);
+        const double c = which == 0 ? c1 : c2;
+        if (c < w.v) { w.v = c; w.i = i0 + 21 * (int64_t)axis; }
+      }
     }
-    const ArgMin r = block_argmin(w, sh);
+    const ArgMin mine = block_argmin(w, sh);
+    if (threadIdx.x == 0) level_best[jj & 1] = mine;
+    cluster.sync();
+    ArgMin r{INFINITY, INT64_MAX};
+    for (int q = 0; q < kRefineCtas; ++q) {
+      const ArgMin o = *cluster.map_shared_rank(&level_best[jj & 1], q);
+      if (better(o, r)) r = o;
+    }
     cur = r.v;
     if (r.i != INT64_MAX) { a[0] = lo[0] + r.i % 21; a[1] = lo[1] + (r.i / 21) % 21; a[2] = lo[2] + r.i / 441; }
     if (fabs(prev - cur) < 1.0e-9 || jj >= 16) break;
     prev = cur;
     jj += 1;
   }
-  if (threadIdx.x == 0) {
+  cluster.sync();   // no CTA leaves while another reads its best
+  if (threadIdx.x == 0 && rank == 0) {
     int64_t* o = ang_out + ((int64_t)dom * 2 + which) * 3;
     o[0] = a[0]; o[1] = a[1]; o[2] = a[2];
     jj_out[dom * 2 + which] = jj;
     crit_out[dom * 2 + which] = cur;
   }
+}
+
+// Two threads per axis while all clusters are resident at once (3 CTAs of 128 threads on each of 148 SMs), where
+// the serial chain of a level counts; one beyond that, where the FP64 pipe does (64 tensors: 1.08 ms
+// with two, 0.77 with one; a single tensor 0.28 with two).
+void launch_refine(const double* ee, const ArgMin* part, int64_t n, int nb, int64_t* ang, int* jj, double* crit,
+                   cudaStream_t s) {
+  const double deg = std::acos(-1.0) / 180.0;
+  const dim3 grid((unsigned)(kRefineCtas * n), 2);
+  if (2 * kRefineCtas * n <= kSweepFill / 2) k_rot_refine<2><<<grid, 2 * kRefineThreads, 0, s>>>(ee, part, nb, deg, ang, jj, crit);
+  else k_rot_refine<1><<<grid, kRefineThreads, 0, s>>>(ee, part, nb, deg, ang, jj, crit);
 }
 
 }  // namespace
@@ -242,7 +379,8 @@ int rotation_search_device(const std::vector<const double*>& ees, std::vector<in
   };
   cudaError_t e;
   if ((e = cudaMalloc(&dee, sizeof(double) * 36 * ndom))) return fail(e, "cudaMalloc");
-  if ((e = cudaMalloc(&dpart, sizeof(ArgMin) * 2 * kSweepBlocks * ndom))) return fail(e, "cudaMalloc");
+  const int nb = sweep_blocks(ndom);
+  if ((e = cudaMalloc(&dpart, sizeof(ArgMin) * 2 * nb * ndom))) return fail(e, "cudaMalloc");
   if ((e = cudaMalloc(&dang, sizeof(int64_t) * 6 * ndom))) return fail(e, "cudaMalloc");
   if ((e = cudaMalloc(&djj, sizeof(int) * 2 * ndom))) return fail(e, "cudaMalloc");
   if ((e = cudaMalloc(&dcrit, sizeof(double) * 2 * ndom))) return fail(e, "cudaMalloc");
@@ -251,8 +389,8 @@ int rotation_search_device(const std::vector<const double*>& ees, std::vector<in
   cudaEvent_t ev[2] = {nullptr, nullptr};
   if (ms && (cudaEventCreate(&ev[0]) != cudaSuccess || cudaEventCreate(&ev[1]) != cudaSuccess)) ms = nullptr;
   if (ms) cudaEventRecord(ev[0], s);
-  k_rot_sweep<<<dim3(kSweepBlocks, ndom), kRotThreads, 0, s>>>(dee, dpart);
-  k_rot_refine<<<dim3(ndom, 2), kRotThreads, 0, s>>>(dee, dpart, std::acos(-1.0) / 180.0, dang, djj, dcrit);
+  k_rot_sweep<<<dim3(nb, ndom), kSweepThreadsRot, 0, s>>>(dee, dpart);
+  launch_refine(dee, dpart, ndom, nb, dang, djj, dcrit, s);
   if (ms) cudaEventRecord(ev[1], s);
   launches += 2;
   if ((e = cudaGetLastError())) {
@@ -315,7 +453,8 @@ extern "C" dtc_status dtc_rotation_search_noalloc(const double* ee, int64_t n, i
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // every block of the sweep writes its own two minima, so no clearing is needed
-  k_rot_sweep<<<dim3(kSweepBlocks, (unsigned)n), kRotThreads, 0, s>>>(ee, part);
-  k_rot_refine<<<dim3((unsigned)n, 2), kRotThreads, 0, s>>>(ee, part, std::acos(-1.0) / 180.0, ang, jj, crit);
+  const int nb = sweep_blocks(n);   // n * nb <= kNoAllocMaxDomains * kSweepBlocks
+  k_rot_sweep<<<dim3(nb, (unsigned)n), kSweepThreadsRot, 0, s>>>(ee, part);
+  launch_refine(ee, part, n, nb, ang, jj, crit, s);
   return cudaGetLastError() == cudaSuccess ? DTC_OK : DTC_ERR_CUDA;
 }
