@@ -13,7 +13,7 @@
 // Work is cut into tiles of 8 x 4 x 4 nodes; a CTA of 128 threads handles one tile for
 // 8 of the 24 load cases (1-D grid, the three load-case groups of a tile adjacent), each
 // thread one (y,z) row of the tile and one load case.  The HEX08 sweeps have their own tiles
-// (sweep.cuh); HEX20 uses voxel bricks (ebe.cuh); the multigrid transfers and the block CG use
+// (sweep.cuh); HEX20 uses voxel columns (hex20.cuh); the multigrid transfers and the block CG use
 // a flat list of active interior nodes (mg.cuh, block.cuh).
 #pragma once
 #include <cstdint>

@@ -3,8 +3,9 @@
 // Operator: the assembled stiffness of the reference (MatSetValues of one Ke per element,
 // f-src/mod_dtc_main_subroutines.f90:516-579) is never formed.  HEX08: K*u is applied
 // matrix-free on voxel rows (sweep.cuh): every kept voxel adds s_v * Khat * u_v to its corners,
-// where s_v = E_v * a and Khat the unit voxel stiffness in its Hadamard basis.  HEX20: element-by-element on voxel bricks staged in shared memory
-// (ebe.cuh), nodes on the doubled grid.  Constrained DOFs (all nodes on the domain box, mod_struct_preprocess.f90:
+// where s_v = E_v * a and Khat the unit voxel stiffness in its Hadamard basis.  HEX20: on voxel columns, in the
+// classes of the reflections
+// (hex20.cuh), nodes on the doubled grid.  Constrained DOFs (all nodes on the domain box, mod_struct_preprocess.f90:
 // 564-592) are excluded from the unknowns exactly like MatZeroRowsColumns with diag 0
 // (:945-951), so the iteration runs on the interior nodes only.
 //
@@ -14,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <map>
@@ -41,7 +43,7 @@ __constant__ double c_k20_64[3600];       // unit HEX20 element matrix (ring nod
 }  // namespace dtc
 
 #include "sweep.cuh"
-#include "ebe.cuh"
+#include "hex20.cuh"
 #include "mg.cuh"
 #include "block.cuh"
 
@@ -57,7 +59,7 @@ template <int NEN> __device__ __forceinline__ int local_node(int ox, int oy, int
 template <> __device__ __forceinline__ int local_node<8>(int ox, int oy, int oz) { return corner_local(ox, oy, oz); }
 template <> __device__ __forceinline__ int local_node<20>(int ox, int oy, int oz) {
   for (int a = 0; a < 20; ++a)
-    if (kRingOff[a][0] == ox && kRingOff[a][1] == oy && kRingOff[a][2] == oz) return a;
+    if (ring_off(a, 0) == ox && ring_off(a, 1) == oy && ring_off(a, 2) == oz) return a;
   return -1;
 }
 template <int NEN> __device__ __forceinline__ double ke64(int i);
@@ -724,6 +726,9 @@ struct DeviceSolver::Impl {
   cudaStream_t stream = nullptr;
   // persistent buffers grown on demand
   std::vector<std::pair<void**, size_t>> owned;
+  // HEX20 unit element matrix of the solve in hand, in its classes
+  ClassBlocks<double> k20_64 = {};
+  ClassBlocks<float> k20_32 = {};
   void* bufs[80] = {nullptr};
   size_t caps[80] = {0};
   // what the solves of the last batch kept for the adjoint: per chunk the domains (node and
@@ -799,7 +804,7 @@ namespace {
 enum Buf { bDoms, bTilesI, bTilesA, bSvox, bFlags, bDinv64, bDinv32, bX, bR64, bP64, bW64, bR32, bX32, bP32, bW32,
            bSt, bOst, bPw, bZz, bZr, bDomAct, bCount, bFf, bTarget, bErr, bBinv32, bBricksI, bBricksA, bZ32, bT32,
            bMgDoms, bMgTiles, bMgSvox, bMgFlags, bMgDinv64, bMgDinv32, bMgBinv32, bMgB, bMgT, bMgZ, bMgMinv, bMgList,
-           bAdjG, bAdjV, bAdjBlk, bAdjGrad, bAdjDoms, bAdjX, bAdjSvox, bKe20, bKe20tc, bNodesI,
+           bAdjG, bAdjV, bAdjBlk, bAdjGrad, bAdjDoms, bAdjX, bAdjSvox, bKe20tc, bBricksTc, bBricksTcC, bNodesI,
            bTilesIc, bNodesIc, bBricksIc, bMgTilesC, bMgListC, bCompactCnt, bMgNodes, bMgNodesC, bXkeep, bTilesW, bTilesWa,
            bTilesWc, bChunks, bChunksC, bNChunk, bBlkSt, bBlkCf, bGram, bGramDone, bNumBufs };
 static_assert(bNumBufs <= 80, "buffer table");
@@ -868,48 +873,49 @@ void launch_ebe_tc(const Tile* bricks, int64_t nb, const DomDev* doms, const flo
 
 namespace {
 
-// CG on one precision: x (interior part), r = b on entry, p = 0 on entry.
-template <typename T, int NEN, bool ALL, bool DOT>
-void launch_ebe(const Tile* bricks, int64_t nb, const DomDev* dd, const float* svox, const uint8_t* fl, const T* ke,
-                const T* u, T* y, double scale, double* acc, const int* act, cudaStream_t s) {
-  using S = EbeShape<T, NEN>;
-  if (nb <= 0) return;
-  k_ebe<T, NEN, ALL, DOT><<<(unsigned)(S::NGRP * nb), S::kThreadsEbe, S::smem, s>>>(bricks, dd, svox, fl, ke, u, y,
-                                                                                    scale, acc, act);
+// One HEX20 application over nt columns of `layers` voxel layers.
+template <typename T, bool ALL, bool DOT>
+void launch_hex20(const Tile* cols, int64_t nt, int layers, const DomDev* dd, const float* svox, const uint8_t* fl,
+                  const ClassBlocks<T>& B, const T* u, T* y, double scale, double* acc, const int* act,
+                  cudaStream_t s) {
+  if (nt <= 0) return;
+  constexpr unsigned groups = kNLC / (kColWords * ColLane<T>::kCols);
+  k_hex20<T, ALL, DOT><<<(unsigned)(groups * nt), kColThreads, kColSmem, s>>>(cols, layers, dd, svox, fl, B, u, y, scale,
+                                                                             acc, act);
 }
 
-template <typename T, int NEN, bool ALL, bool DOT>
-int allow_ebe_smem(std::string& msg) {
-  DTC_CUDA(cudaFuncSetAttribute(k_ebe<T, NEN, ALL, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)EbeShape<T, NEN>::smem));
+template <typename T, bool ALL, bool DOT>
+int allow_hex20_smem(std::string& msg) {
+  DTC_CUDA(cudaFuncSetAttribute(k_hex20<T, ALL, DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kColSmem));
   return DTC_OK;
 }
 
-template <int NEN>
-int allow_all_ebe(std::string& msg) {
+int allow_all_hex20(std::string& msg) {
   int e;
-  if ((e = allow_ebe_smem<float, NEN, false, true>(msg))) return e;
-  if ((e = allow_ebe_smem<float, NEN, false, false>(msg))) return e;   // multigrid residual sweeps
-  if ((e = allow_ebe_smem<double, NEN, false, true>(msg))) return e;
-  if ((e = allow_ebe_smem<double, NEN, false, false>(msg))) return e;
-  if ((e = allow_ebe_smem<double, NEN, true, false>(msg))) return e;
-  return DTC_OK;
+  if ((e = allow_hex20_smem<float, false, true>(msg))) return e;
+  if ((e = allow_hex20_smem<float, false, false>(msg))) return e;   // multigrid residual sweeps
+  if ((e = allow_hex20_smem<double, false, true>(msg))) return e;
+  if ((e = allow_hex20_smem<double, false, false>(msg))) return e;
+  return allow_hex20_smem<double, true, false>(msg);
 }
 
 // Work lists of one solve: node tiles (vector kernels and the HEX08 node-centric operator)
-// and voxel bricks (HEX20 element-by-element operator), over the interior / all nodes.
+// and voxel columns (HEX20 operator), over the interior / all nodes.
 struct Work {
   const Tile *ti, *ta, *bi, *ba;
   int64_t nti, nta, nbi, nba;
   const int64_t* nodes;  // active interior nodes, (domain << kListShift) | node
   int64_t nnodes;
-  const double* ke64;   // HEX20 unit element matrix (FP64, then its FP32 copy)
-  const float* ke32;
+  const ClassBlocks<double>* ke64;   // HEX20 unit element matrix in its classes (host memory)
+  const ClassBlocks<float>* ke32;
+  int layers;           // voxel layers of a HEX20 column
   const float* ke20tc;  // HEX20 FP32 applications on tcgen05: split matrix in the B layout, else null
   int* err;             // mbarrier time-out flag of the tensor-core kernels
   const Tile *tw = nullptr, *twa = nullptr;   // tiles of the HEX08 sweeps over the interior / all nodes
   int64_t ntw = 0, ntwa = 0;
   int len = kSweepX;               // their nodes in x
+  const Tile* bt = nullptr;        // voxel bricks of the HEX20 operator on tcgen05, interior
+  int64_t nbt = 0;
   const Chunk* chunks = nullptr;   // the node list in pieces of one domain (CG vector kernels)
   int64_t nchunks = 0;
 };
@@ -948,16 +954,17 @@ void apply_k(const Work& W, const DomDev* dd, const float* svox, const uint8_t* 
     launch_sweep<T, ALL, DOT ? kSwApplyDot : kSwApply>(ALL ? W.ntwa : W.ntw, W.len, s, ALL ? W.twa : W.tw, dd, svox,
                                                        u, y, scale, nullptr, nullptr, 0.f, acc, act);
   } else {
-    const T* ke;
-    if constexpr (sizeof(T) == 8) ke = W.ke64;
-    else ke = W.ke32;
     if constexpr (sizeof(T) == 4 && !ALL) {
       if (W.ke20tc) {
-        launch_ebe_tc(W.bi, W.nbi, dd, svox, fl, W.ke20tc, u, y, scale, DOT ? acc : nullptr, act, W.err, s);
+        launch_ebe_tc(W.bt, W.nbt, dd, svox, fl, W.ke20tc, u, y, scale, DOT ? acc : nullptr, act, W.err, s);
         return;
       }
     }
-    launch_ebe<T, NEN, ALL, DOT>(ALL ? W.ba : W.bi, ALL ? W.nba : W.nbi, dd, svox, fl, ke, u, y, scale, acc, act, s);
+    const ClassBlocks<T>* ke;
+    if constexpr (sizeof(T) == 8) ke = W.ke64;
+    else ke = W.ke32;
+    launch_hex20<T, ALL, DOT>(ALL ? W.ba : W.bi, ALL ? W.nba : W.nbi, W.layers, dd, svox, fl, *ke, u, y, scale, acc, act,
+                              s);
   }
 }
 
@@ -975,6 +982,24 @@ int sweep_length(int64_t tiles) {
   int len = kSweepX;
   while (len > 4 && 3 * tiles * (kSweepX / len) < 2 * 148) len /= 2;
   return len;
+}
+
+// Voxel layers of the HEX20 columns over grids of these voxels per edge: a CTA that starts above the lowest layer
+// evaluates one layer more than it owns, and an SM holds one CTA, so the length is the one whose longest SM (three
+// groups of load cases, 148 SMs) has the fewest layers to walk.
+int hex20_layers(const std::vector<std::array<int, 3>>& grids) {
+  auto up = [](int n, int t) { return (int64_t)((n + t - 1) / t); };
+  int most = 1;
+  for (const auto& L : grids) most = std::max(most, L[2]);
+  int best = most;
+  int64_t cost = INT64_MAX;
+  for (int len = most; len >= 1; --len) {
+    int64_t ctas = 0;
+    for (const auto& L : grids) ctas += 3 * up(L[0], kColX) * up(L[1], kColY) * up(L[2], len);
+    const int64_t c = (ctas + 147) / 148 * (len + 1);
+    if (c < cost) { cost = c; best = len; }
+  }
+  return best;
 }
 
 // Multigrid hierarchy of one solve (HEX08, FP32 inner solve).  Level 0 is the fine grid
@@ -1322,12 +1347,15 @@ struct MgDev {
   float *b, *t, *z;      // levels >= 1
   float *t0, *z0;        // fine level
   int nen0;              // element of the fine level; HEX20 applies K with the brick kernel
-  const Tile* bricks0;   // fine-level interior bricks (HEX20)
+  const Tile* bricks0;   // fine-level interior columns (HEX20) and, for the tensor cores, bricks
   int64_t nbricks0;
+  int layers0;           // voxel layers of a column
+  const Tile* tcbricks0;
+  int64_t ntcbricks0;
   const int64_t* nodes0; // fine-level active interior nodes, (domain << kListShift) | node
   int64_t nnodes0;
-  const float* ke32;     // HEX20 unit element matrix (FP32)
-  const float* ke20tc;   // its tensor-core operand, or null (brick SIMT kernel)
+  const ClassBlocks<float>* ke32;   // HEX20 unit element matrix in its classes (host memory)
+  const float* ke20tc;   // its tensor-core operand, or null (SIMT kernel)
   int* err;
 };
 
@@ -1396,9 +1424,9 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   }
   if (fine && M.nen0 == 20) {
     if (M.ke20tc)
-      launch_ebe_tc(M.bricks0, M.nbricks0, dl, sv, fl, M.ke20tc, t, z, -1.0, nullptr, act, M.err, s);
+      launch_ebe_tc(M.tcbricks0, M.ntcbricks0, dl, sv, fl, M.ke20tc, t, z, -1.0, nullptr, act, M.err, s);
     else
-      launch_ebe<float, 20, false, false>(M.bricks0, M.nbricks0, dl, sv, fl, M.ke32, t, z, -1.0, nullptr, act, s);
+      launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, dl, sv, fl, *M.ke32, t, z, -1.0, nullptr, act, s);
     k_mg_combine<kMgRes><<<g, kThreads, 0, s>>>(tsm, dl, fl, bi, b, t, z, om, act);
     ++launches;
   } else if (fine && I.tensor_matvec) {
@@ -1433,9 +1461,9 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   q = fine ? I.begin(0) : -1;
   if (l == 0 && M.nen0 == 20) {
     if (M.ke20tc)
-      launch_ebe_tc(M.bricks0, M.nbricks0, dl, sv, fl, M.ke20tc, t, z, -1.0, nullptr, act, M.err, s);
+      launch_ebe_tc(M.tcbricks0, M.ntcbricks0, dl, sv, fl, M.ke20tc, t, z, -1.0, nullptr, act, M.err, s);
     else
-      launch_ebe<float, 20, false, false>(M.bricks0, M.nbricks0, dl, sv, fl, M.ke32, t, z, -1.0, nullptr, act, s);
+      launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, dl, sv, fl, *M.ke32, t, z, -1.0, nullptr, act, s);
     k_mg_combine<kMgPost><<<g, kThreads, 0, s>>>(tsm, dl, fl, bi, b, t, z, P.omega0, act);
     ++launches;
   } else if (l == 0 && I.tensor_matvec)
@@ -1539,13 +1567,14 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   cudaStream_t s = I.stream;
   static const MgPlan kNoLevels;
   const MgPlan& P = M ? *M->P : kNoLevels;
-  const int nseg = 5 + 5 * P.nlev;
+  const int nseg = 6 + 5 * P.nlev;
   int e;
   if ((e = ensure(I, bCompactCnt, sizeof(int) * nseg, msg))) return e;
   if ((e = ensure(I, bTilesIc, sizeof(Tile) * std::max<int64_t>(W.nti, 1), msg))) return e;
   if ((e = ensure(I, bTilesWc, sizeof(Tile) * std::max<int64_t>(W.ntw, 1), msg))) return e;
   if ((e = ensure(I, bNodesIc, sizeof(int64_t) * std::max<int64_t>(W.nnodes, 1), msg))) return e;
   if ((e = ensure(I, bBricksIc, sizeof(Tile) * std::max<int64_t>(W.nbi, 1), msg))) return e;
+  if ((e = ensure(I, bBricksTcC, sizeof(Tile) * std::max<int64_t>(W.nbt, 1), msg))) return e;
   if ((e = ensure(I, bChunksC, sizeof(Chunk) * std::max<int64_t>(W.nchunks, 1), msg))) return e;
   if ((e = ensure(I, bMgTilesC, sizeof(Tile) * std::max<size_t>(P.tiles.size(), 1), msg))) return e;
   if ((e = ensure(I, bMgListC, sizeof(int) * std::max<size_t>(P.lists.size(), 1), msg))) return e;
@@ -1556,6 +1585,7 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   Tile* wc = B<Tile>(I, bTilesWc);
   int64_t* nc = B<int64_t>(I, bNodesIc);
   Tile* bc = B<Tile>(I, bBricksIc);
+  Tile* bt = B<Tile>(I, bBricksTcC);
   Tile* mt = B<Tile>(I, bMgTilesC);
   int* ml = B<int>(I, bMgListC);
   int64_t* mn = B<int64_t>(I, bMgNodesC);
@@ -1565,12 +1595,13 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   launch_compact(W.bi, W.nbi, act, bc, cnt + 2, s);
   launch_compact(W.tw, W.ntw, act, wc, cnt + 3, s);
   launch_compact(W.chunks, W.nchunks, act, cc, cnt + 4, s);
+  launch_compact(W.bt, W.nbt, act, bt, cnt + 5, s);
   for (int l = 0; l < P.nlev; ++l) {
-    launch_compact(M->tiles + P.sm_off[l], P.sm_n[l], act, mt + P.sm_off[l], cnt + 5 + 5 * l, s);
-    launch_compact(M->tiles + P.in_off[l], P.in_n[l], act, mt + P.in_off[l], cnt + 6 + 5 * l, s);
-    launch_compact(M->lists + P.list_off[l], P.list_n[l], act, ml + P.list_off[l], cnt + 7 + 5 * l, s);
-    launch_compact(M->nodes + P.nl_off[l], P.nl_n[l], act, mn + P.nl_off[l], cnt + 8 + 5 * l, s);
-    launch_compact(M->tiles + P.sw_off[l], P.sw_n[l], act, mt + P.sw_off[l], cnt + 9 + 5 * l, s);
+    launch_compact(M->tiles + P.sm_off[l], P.sm_n[l], act, mt + P.sm_off[l], cnt + 6 + 5 * l, s);
+    launch_compact(M->tiles + P.in_off[l], P.in_n[l], act, mt + P.in_off[l], cnt + 7 + 5 * l, s);
+    launch_compact(M->lists + P.list_off[l], P.list_n[l], act, ml + P.list_off[l], cnt + 8 + 5 * l, s);
+    launch_compact(M->nodes + P.nl_off[l], P.nl_n[l], act, mn + P.nl_off[l], cnt + 9 + 5 * l, s);
+    launch_compact(M->tiles + P.sw_off[l], P.sw_n[l], act, mt + P.sw_off[l], cnt + 10 + 5 * l, s);
   }
   launches += nseg;
   if ((e = launch_check(msg))) return e;
@@ -1582,18 +1613,20 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   Wc.bi = bc; Wc.nbi = h[2];
   Wc.tw = wc; Wc.ntw = h[3];
   Wc.chunks = cc; Wc.nchunks = h[4];
+  Wc.bt = bt; Wc.nbt = h[5];
   if (M) {
     Mc->bricks0 = bc; Mc->nbricks0 = h[2];
+    Mc->tcbricks0 = bt; Mc->ntcbricks0 = h[5];
     Mc->nodes0 = nc; Mc->nnodes0 = h[1];
     Mc->tiles = mt;
     Mc->lists = ml;
     Mc->nodes = mn;
     for (int l = 0; l < P.nlev; ++l) {
-      Pc->sm_n[l] = h[5 + 5 * l];
-      Pc->in_n[l] = h[6 + 5 * l];
-      Pc->list_n[l] = h[7 + 5 * l];
-      Pc->nl_n[l] = h[8 + 5 * l];
-      Pc->sw_n[l] = h[9 + 5 * l];
+      Pc->sm_n[l] = h[6 + 5 * l];
+      Pc->in_n[l] = h[7 + 5 * l];
+      Pc->list_n[l] = h[8 + 5 * l];
+      Pc->nl_n[l] = h[9 + 5 * l];
+      Pc->sw_n[l] = h[10 + 5 * l];
     }
   }
   return DTC_OK;
@@ -1847,7 +1880,7 @@ TuneKey tune_key(int device, int nen, const std::vector<DomDev>& doms, const std
 // class (median domain edge in quarter octaves, kept-voxel fraction below 0.15 / 0.30 / above)
 // by CUDA-event timings on the batch's own tiles and vectors:
 //  * HEX08: the SIMT sweep or the tcgen05 sweep (timed on the post-smoothing sweep);
-//  * HEX20: the SIMT brick kernel or the tcgen05 brick kernel (the operator of the residual and
+//  * HEX20: the SIMT column kernel or the tcgen05 brick kernel (the operator of the residual and
 //    post-smoothing steps and of the CG application).
 int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, const std::vector<DomDev>& doms,
                    const std::vector<float>& svox, int nen, std::string& msg) {
@@ -1867,7 +1900,7 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
   }
   const int64_t nsm = M.P->sm_n[0];
   const Tile* tsm = M.tiles + M.P->sm_off[0];
-  if (nsm <= 0 || (nen == 20 && (M.nbricks0 <= 0 || !W.ke20tc))) return DTC_OK;
+  if (nsm <= 0 || (nen == 20 && (M.ntcbricks0 <= 0 || !W.ke20tc))) return DTC_OK;
   const float* b = B<float>(I, bR32);
   const Tile* tsw = M.tiles + M.P->sw_off[0];
   const int64_t gw = M.P->sw_n[0];
@@ -1878,10 +1911,10 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
     auto launch = [&]() {
       if (nen == 20) {
         if (cand == 0)
-          launch_ebe<float, 20, false, false>(M.bricks0, M.nbricks0, M.doms0, M.svox0, M.flags0, M.ke32, M.t0, M.z0,
-                                              -1.0, nullptr, nullptr, s);
+          launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, M.doms0, M.svox0, M.flags0, *M.ke32, M.t0,
+                                            M.z0, -1.0, nullptr, nullptr, s);
         else
-          launch_ebe_tc(M.bricks0, M.nbricks0, M.doms0, M.svox0, M.flags0, W.ke20tc, M.t0, M.z0, -1.0, nullptr,
+          launch_ebe_tc(M.tcbricks0, M.ntcbricks0, M.doms0, M.svox0, M.flags0, W.ke20tc, M.t0, M.z0, -1.0, nullptr,
                         nullptr, M.err, s);
       } else if (cand == 0) {
         launch_mg_matvec<kMgPost>(gw, sl, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
@@ -1903,7 +1936,8 @@ struct HostBatch {
   int nen = 0;
   std::vector<int64_t> tidx;   // tasks solved in this pass
   std::vector<DomDev> doms;
-  std::vector<Tile> tiles_i, tiles_a, bricks_i, bricks_a;
+  std::vector<Tile> tiles_i, tiles_a, bricks_i, bricks_a, bricks_t;
+  int layers = 1;              // voxel layers of a HEX20 column
   std::vector<Tile> tiles_w, tiles_wa;   // sweep tiles (HEX08) over the interior / all nodes
   int sweep_len = kSweepX;               // their nodes in x
   std::vector<int64_t> nodes_i;
@@ -1936,6 +1970,7 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
   const int ndom_p = (int)tidx.size();
   std::vector<int64_t> vox_offs(ndom_p), node_offs(ndom_p);
   int64_t vox_total = 0, sweep_total = 0;
+  std::vector<std::array<int, 3>> grids;
   for (int d = 0; d < ndom_p; ++d) {
     const dtc_domain_in& in = *tasks[tidx[d]].in;
     vox_offs[d] = vox_total;
@@ -1943,15 +1978,18 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
     vox_total += in.L[0] * in.L[1] * in.L[2];
     const int L[3] = {(int)in.L[0], (int)in.L[1], (int)in.L[2]};
     sweep_total += sweep_tiles(L);
+    grids.push_back({L[0], L[1], L[2]});
     node_total += (int64_t)(m * in.L[0] + 1) * (m * in.L[1] + 1) * (m * in.L[2] + 1);
   }
   hb.sweep_len = sweep_length(sweep_total);
+  if (NEN == 20) hb.layers = hex20_layers(grids);
+  const bool bricks_tc = opt.precision == DTC_PREC_MIXED && opt.mixed_matvec != 0;
   const int len = hb.sweep_len;
   svox.assign((size_t)vox_total, 0.f);
   // per domain: voxel factors, node activity and work lists (host threads)
   struct Packed {
     DomDev D;
-    std::vector<Tile> ti, ta, bi, ba, tw, twa;
+    std::vector<Tile> ti, ta, bi, ba, bt, tw, twa;
     std::vector<int64_t> ni;
     double vec = 0, mv = 0, fl = 0;
   };
@@ -2045,16 +2083,20 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
         for (int x0 = 0; x0 <= nx - 1; x0 += kTileX)
           if (any_active(x0, y0, z0, kTileX, kTileY, kTileZ, 0, nx - 1, ny - 1, nz - 1))
             out.ta.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
-    // voxel bricks (HEX20 operator): brick origin in voxels, owned nodes m*origin + [0, m*B)
-    for (int bz = 0; NEN == 20 && m * bz <= nz - 1; bz += EL::BZ)
-      for (int by = 0; m * by <= ny - 1; by += EL::BY)
-        for (int bx = 0; m * bx <= nx - 1; bx += EL::BX) {
-          const int ox = m * bx, oy = m * by, oz = m * bz;
-          if (any_active(ox, oy, oz, m * EL::BX, m * EL::BY, m * EL::BZ, 1, nx - 2, ny - 2, nz - 2))
-            out.bi.push_back(Tile{dom, (int16_t)bx, (int16_t)by, (int16_t)bz, 0});
-          if (any_active(ox, oy, oz, m * EL::BX, m * EL::BY, m * EL::BZ, 0, nx - 1, ny - 1, nz - 1))
-            out.ba.push_back(Tile{dom, (int16_t)bx, (int16_t)by, (int16_t)bz, 0});
-        }
+    // HEX20 operator: voxel columns, and voxel bricks for its form on the tensor cores; the origin is in voxels,
+    // the owned nodes are 2 * origin + [0, 2 * size)
+    auto list20 = [&](std::vector<Tile>& to, int sx, int sy, int sz, int lo, int hx, int hy, int hz) {
+      for (int bz = 0; 2 * bz <= nz - 1; bz += sz)
+        for (int by = 0; 2 * by <= ny - 1; by += sy)
+          for (int bx = 0; 2 * bx <= nx - 1; bx += sx)
+            if (any_active(2 * bx, 2 * by, 2 * bz, 2 * sx, 2 * sy, 2 * sz, lo, hx, hy, hz))
+              to.push_back(Tile{dom, (int16_t)bx, (int16_t)by, (int16_t)bz, 0});
+    };
+    if (NEN == 20) {
+      list20(out.bi, kColX, kColY, hb.layers, 1, nx - 2, ny - 2, nz - 2);
+      list20(out.ba, kColX, kColY, hb.layers, 0, nx - 1, ny - 1, nz - 1);
+      if (bricks_tc) list20(out.bt, 4, 4, 2, 1, nx - 2, ny - 2, nz - 2);
+    }
     out.D = D;
   };
   parallel_for(ndom_p, opt.host_threads, [&](int64_t d) { pack_one((int)d, packed[d]); });
@@ -2076,6 +2118,7 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
     hb.tiles_wa.insert(hb.tiles_wa.end(), q.twa.begin(), q.twa.end());
     bricks_i.insert(bricks_i.end(), q.bi.begin(), q.bi.end());
     bricks_a.insert(bricks_a.end(), q.ba.begin(), q.ba.end());
+    hb.bricks_t.insert(hb.bricks_t.end(), q.bt.begin(), q.bt.end());
     nodes_i.insert(nodes_i.end(), q.ni.begin(), q.ni.end());
     hb.dom_vec.push_back(q.vec);
     hb.dom_mv.push_back(q.mv);
@@ -2131,15 +2174,10 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
     }
     if (NEN == 20) {
       std::vector<double> k20(3600);
-      std::vector<float> k20f(3600);
       voxel_stiffness(20, nu, k20.data());
-      for (int i = 0; i < 3600; ++i) k20f[i] = (float)k20[i];
       DTC_CUDA(cudaMemcpyToSymbolAsync(c_k20_64, k20.data(), sizeof(double) * 3600, 0, cudaMemcpyHostToDevice, s));
-      // the element kernel stages the matrix from global memory: FP64 then FP32 copy
-      if (int e = ensure(I, bKe20, sizeof(double) * 3600 + sizeof(float) * 3600, msg)) return e;
-      DTC_CUDA(cudaMemcpyAsync(I.bufs[bKe20], k20.data(), sizeof(double) * 3600, cudaMemcpyHostToDevice, s));
-      DTC_CUDA(cudaMemcpyAsync(B<double>(I, bKe20) + 3600, k20f.data(), sizeof(float) * 3600, cudaMemcpyHostToDevice,
-                               s));
+      I.k20_64 = class_blocks<double>(k20.data());
+      I.k20_32 = class_blocks<float>(k20.data());
       if (I.tensor_matvec || tune) {   // HEX20 FP32 applications on the tensor cores
         std::vector<float> img(tc20_operand_bytes() / sizeof(float));
         build_tc20_operand(k20.data(), img.data());
@@ -2150,8 +2188,8 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
       DTC_CUDA(cudaStreamSynchronize(s));   // the host vectors go out of scope
     }
     if (int e = allow_all_sweeps(msg)) return e;   // per device, cheap
-    if constexpr (NEN == 20)
-      if (int e = allow_all_ebe<NEN>(msg)) return e;
+    if (NEN == 20)
+      if (int e = allow_all_hex20(msg)) return e;
   }
   // the host side of the pass (prepare_nen)
   const auto tpack = std::chrono::steady_clock::now();
@@ -2184,6 +2222,8 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   const int64_t ntwa = (int64_t)hb.tiles_wa.size();
   if ((e = ensure(I, bTilesWa, sizeof(Tile) * std::max<int64_t>(ntwa, 1), msg))) return e;
   if ((e = ensure(I, bBricksI, sizeof(Tile) * std::max<int64_t>(nbi, 1), msg))) return e;
+  const int64_t nbt = (int64_t)hb.bricks_t.size();
+  if ((e = ensure(I, bBricksTc, sizeof(Tile) * std::max<int64_t>(nbt, 1), msg))) return e;
   if ((e = ensure(I, bBricksA, sizeof(Tile) * std::max<int64_t>(nba, 1), msg))) return e;
   I.svox_dev = nullptr;
   if (hb.up_slot < 0 && (e = ensure(I, bSvox, sizeof(float) * svox.size(), msg))) return e;
@@ -2243,6 +2283,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   if (!hb.chunks.empty())
     DTC_CUDA(cudaMemcpyAsync(I.bufs[bChunks], hb.chunks.data(), sizeof(Chunk) * hb.chunks.size(),
                              cudaMemcpyHostToDevice, s));
+  if (nbt) DTC_CUDA(cudaMemcpyAsync(I.bufs[bBricksTc], hb.bricks_t.data(), sizeof(Tile) * nbt, cudaMemcpyHostToDevice, s));
   if (nba) DTC_CUDA(cudaMemcpyAsync(I.bufs[bBricksA], bricks_a.data(), sizeof(Tile) * nba, cudaMemcpyHostToDevice, s));
   if (hb.up_slot >= 0) {   // uploaded while the previous pass solved: order the solve after the copy
     DTC_CUDA(cudaStreamWaitEvent(s, I.up_ev[hb.up_slot], 0));
@@ -2264,11 +2305,12 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   }
   const Tile* ti = B<Tile>(I, bTilesI);
   const Tile* ta = B<Tile>(I, bTilesA);
-  const double* ke64 = NEN == 20 ? B<double>(I, bKe20) : nullptr;
   const float* ke20tc = (NEN == 20 && (I.tensor_matvec || tune)) ? B<float>(I, bKe20tc) : nullptr;
   Work W{ti, ta, B<Tile>(I, bBricksI), B<Tile>(I, bBricksA), nti, nta, nbi, nba,
-               B<int64_t>(I, bNodesI), (int64_t)nodes_i.size(), ke64,
-               ke64 ? reinterpret_cast<const float*>(ke64 + 3600) : nullptr, ke20tc, B<int>(I, bErr)};
+               B<int64_t>(I, bNodesI), (int64_t)nodes_i.size(), &I.k20_64,
+               &I.k20_32, hb.layers, ke20tc, B<int>(I, bErr)};
+  W.bt = B<Tile>(I, bBricksTc);
+  W.nbt = nbt;
   W.tw = B<Tile>(I, bTilesW);
   W.ntw = ntw;
   W.twa = B<Tile>(I, bTilesWa);
@@ -2376,6 +2418,9 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
     mgd.nen0 = NEN;
     mgd.bricks0 = W.bi;
     mgd.nbricks0 = W.nbi;
+    mgd.layers0 = W.layers;
+    mgd.tcbricks0 = W.bt;
+    mgd.ntcbricks0 = W.nbt;
     mgd.nodes0 = W.nodes;
     mgd.nnodes0 = W.nnodes;
     mgd.ke32 = W.ke32;
@@ -2383,7 +2428,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
     mgd.err = W.err;
     if (tune) {
       if ((e = autotune_sweep(I, stats_, W, mgd, doms, svox, NEN, msg))) return e;
-      if (!I.tensor_matvec) W.ke20tc = mgd.ke20tc = nullptr;   // HEX20: the brick kernel won
+      if (!I.tensor_matvec) W.ke20tc = mgd.ke20tc = nullptr;   // HEX20: the column kernel won
       // the timed launches wrote the fine multigrid vectors
       DTC_CUDA(cudaMemsetAsync(I.bufs[bZ32], 0, vbytes32, s));
       DTC_CUDA(cudaMemsetAsync(I.bufs[bT32], 0, vbytes32, s));

@@ -466,7 +466,7 @@ int upload_tc_operand(const double* khat, cudaStream_t s, std::string& msg) {
 }
 
 // -------------------------------------------------------------------------------------
-// HEX20: the 60x60 element contraction of the brick kernel (ebe.cuh) on the tensor cores.
+// HEX20: the 60x60 element contraction on voxel bricks of 4 x 4 x 2 on the tensor cores.
 namespace tc20 {
 constexpr int kRows = 128, kVoxPerRound = 32, kLcg = 4;
 constexpr int kK = 64, kN = 64, kKc = 8, kChunks = kK / kKc;
