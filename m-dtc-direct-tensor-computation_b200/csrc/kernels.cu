@@ -34,6 +34,7 @@
 namespace dtc {
 
 __constant__ double c_khat64[576];   // unit voxel stiffness, column-major (symmetric)
+__constant__ float c_kh32[576];      // the same in FP32 (k_mg_tail)
 // the 24 load-case columns of the current column pass of the macro modes for eps = 1e-6:
 // uu(nm,3,24) column-major, nm = 8 (macro order 1) or 20 (macro order 2); columns past the
 // last load case are zero
@@ -937,6 +938,7 @@ int allow_sweep_smem(std::string& msg) {
 }
 int allow_all_sweeps(std::string& msg) {
   int e;
+  DTC_CUDA(cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
   if ((e = allow_sweep_smem<float, false, kSwApply>(msg))) return e;
   if ((e = allow_sweep_smem<float, false, kSwApplyDot>(msg))) return e;
   if ((e = allow_sweep_smem<float, false, kSwRes>(msg))) return e;
@@ -1019,7 +1021,9 @@ struct MgPlan {
   std::vector<int> lists;
   std::vector<int64_t> list_off, list_n;
   std::vector<int64_t> nodes_l;                     // levels >= 1: active interior nodes, (domain << kListShift) | node
-  std::vector<int64_t> nl_off, nl_n;
+  std::vector<int64_t> nl_off, nl_n;                // of the domains that take part as kernels of their own: restriction
+  std::vector<int64_t> ns_off, ns_n;                // targets, and those that smooth on the level
+  bool tail = false;                                // the last two levels (not the finest) in one kernel, k_mg_tail
   std::vector<float> svox;                          // voxels of levels >= 1
   std::vector<float> minv;                          // ndom * 81 * 81
   int64_t nodes = 0;                                // nodes of levels >= 1
@@ -1151,6 +1155,10 @@ void coarse_inverse(const DomDev& D, const float* sv, const double* kh, float* o
 // uneven batch (16^3-64^3) ~3.5% less solve time than once everywhere; twice already on
 // level 1 costs more than the iterations it saves.
 constexpr int kMgTwiceFrom = 2;
+// Most domains of a solve whose last two levels run as one kernel (six CTAs a domain, one at a time on an SM): the
+// coarse levels of 64 domains of 32^3 take 18.1 ms of a solve instead of 21.4, of 128 28.7 instead of 30.1, of
+// 192 40.8 and 40.3, of 384 80.9 and 77.9, where the sweeps' fewer operations count.
+constexpr int kTailDomains = 128;
 
 // HEX20 fine grids (m = 2) get one p-coarsening first: level 1 is the HEX08 mesh of the same
 // voxels (corner nodes; the trilinear space is contained in the serendipity one, so the
@@ -1183,12 +1191,13 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
     }
     nl = std::max(nl, nlev[d]);
   }
+  P.tail = ndom <= kTailDomains;
   // nodes in x of the levels' sweep tiles
   P.sw_len.assign(nl, fine_len);
   for (int l = 1; l < nl; ++l) {
     int64_t tiles = 0;
     for (int d = 0; d < ndom; ++d) {
-      if (nlev[d] <= l + 1) continue;
+      if (nlev[d] <= l + 1 + P.tail) continue;
       int n[3];
       for (int k = 0; k < 3; ++k) {
         n[k] = doms0[d].L[k];
@@ -1255,14 +1264,14 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
             if (any(x0, y0, z0, 1, nx - 2, ny - 2, nz - 2)) {
               const Tile t{d, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0};
               Lv.t_in.push_back(t);
-              if (nlev[d] > l + 1) Lv.t_sm.push_back(t);
+              if (nlev[d] > l + 1 + P.tail) Lv.t_sm.push_back(t);
             }
       for (int z0 = 0; z0 <= nz - 1; z0 += kTileZ)
         for (int y0 = 0; y0 <= ny - 1; y0 += kTileY)
           for (int x0 = 0; x0 <= nx - 1; x0 += kTileX)
             if (any(x0, y0, z0, 0, nx - 1, ny - 1, nz - 1))
               Lv.t_all.push_back(Tile{d, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
-      if (nlev[d] > l + 1)
+      if (nlev[d] > l + 1 + P.tail)
         for (int z0 = 1; z0 <= nz - 2; z0 += kSweepZ)
           for (int y0 = 1; y0 <= ny - 2; y0 += kSweepY)
             for (int x0 = 1; x0 <= nx - 2; x0 += P.sw_len[l])
@@ -1289,7 +1298,7 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
   P.sm_off.assign(nl, 0); P.sm_n.assign(nl, 0); P.in_off.assign(nl, 0); P.in_n.assign(nl, 0);
   P.sw_off.assign(nl, 0); P.sw_n.assign(nl, 0);
   P.all_off.assign(nl, 0); P.all_n.assign(nl, 0); P.list_off.assign(nl, 0); P.list_n.assign(nl, 0);
-  P.nl_off.assign(nl, 0); P.nl_n.assign(nl, 0);
+  P.nl_off.assign(nl, 0); P.nl_n.assign(nl, 0); P.ns_off.assign(nl, 0); P.ns_n.assign(nl, 0);
   P.tiles.clear(); P.lists.clear(); P.svox.clear(); P.nodes_l.clear(); P.nodes = 0;
   for (int d = 0; d < ndom; ++d) P.doms[d] = doms0[d];
   P.sm_off[0] = 0;
@@ -1318,12 +1327,16 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
     append(&Level::t_in, P.in_off[l], P.in_n[l]);
     append(&Level::t_all, P.all_off[l], P.all_n[l]);
     append(&Level::t_sw, P.sw_off[l], P.sw_n[l]);
-    P.nl_off[l] = (int64_t)P.nodes_l.size();
-    for (int d = 0; d < ndom; ++d)
-      if (nlev[d] > l)
-        for (const int32_t k : lev[d][l].n_in)
-          P.nodes_l.push_back(((int64_t)d << kListShift) | (lev[d][l].C.node_off + k));
-    P.nl_n[l] = (int64_t)P.nodes_l.size() - P.nl_off[l];
+    auto append_nodes = [&](auto&& takes, int64_t& off, int64_t& cnt) {
+      off = (int64_t)P.nodes_l.size();
+      for (int d = 0; d < ndom; ++d)
+        if (takes(nlev[d]))
+          for (const int32_t k : lev[d][l].n_in)
+            P.nodes_l.push_back(((int64_t)d << kListShift) | (lev[d][l].C.node_off + k));
+      cnt = (int64_t)P.nodes_l.size() - off;
+    };
+    append_nodes([&](int n) { return n > l + 1 || (n == l + 1 && (l == 1 || !P.tail)); }, P.nl_off[l], P.nl_n[l]);
+    append_nodes([&](int n) { return n > l + 1 + P.tail; }, P.ns_off[l], P.ns_n[l]);
   }
   for (int l = 0; l < nl; ++l) {
     P.list_off[l] = (int64_t)P.lists.size();
@@ -1385,8 +1398,14 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   const double mb = I.profile && fine ? I.active_sum(I.dom_mv_bytes) * sizeof(float) : 0;
   const double mf = I.profile && fine ? I.active_sum(I.dom_mv_flops) : 0;
   const int q0 = fine ? -1 : I.begin(0);
-  if (P.list_n[l] > 0) {
+  if (P.list_n[l] > 0 && (l <= 1 || !P.tail)) {
     k_mg_coarse<<<(unsigned)P.list_n[l], kMgCoarseThreads, 0, s>>>(M.lists + P.list_off[l], dl, M.minv, b, z, act);
+    ++launches;
+  }
+  if (!fine && P.tail && l + 1 < P.nlev && P.list_n[l + 1] > 0) {
+    k_mg_tail<<<(unsigned)(kNLC / kTailLc * P.list_n[l + 1]), kTailThreads, kTailSmem, s>>>(
+        M.lists + P.list_off[l + 1], dl, M.doms + (size_t)(l + 1) * M.ndom, sv, fl, bi, M.minv, b, z, P.omega,
+        l >= kMgTwiceFrom ? 4 : 2, act);
     ++launches;
   }
   const int64_t nsm = P.sm_n[l];
@@ -1402,9 +1421,9 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   int q = -1;
   if (!(fine && t_ready)) {
     q = fine ? I.begin(0) : -1;
-    const int64_t items = (int64_t)kQuads * (fine ? M.nnodes0 : P.nl_n[l]);
+    const int64_t items = (int64_t)kQuads * (fine ? M.nnodes0 : P.ns_n[l]);
     if (items > 0)
-      k_mg_jacobi_flat<<<(unsigned)((items + 255) / 256), 256, 0, s>>>(fine ? M.nodes0 : M.nodes + P.nl_off[l], items,
+      k_mg_jacobi_flat<<<(unsigned)((items + 255) / 256), 256, 0, s>>>(fine ? M.nodes0 : M.nodes + P.ns_off[l], items,
                                                                          M.doms + (size_t)(l + 1) * M.ndom, bi, b,
                                                                          fine ? P.omega0 : P.omega, t, act);
     if (fine) I.end(kcMgJacobi, q, 2 * vb + vb / 12, 0);   // b in, t out, 6 floats of D^-1 per node
@@ -1452,9 +1471,9 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   const int q1 = fine ? -1 : I.begin(0);
   q = fine ? I.begin(0) : -1;
   {
-    const int64_t items = (int64_t)kQuads * (fine ? M.nnodes0 : P.nl_n[l]);
+    const int64_t items = (int64_t)kQuads * (fine ? M.nnodes0 : P.ns_n[l]);
     if (items > 0)
-      k_mg_prolong_flat<<<(unsigned)((items + 255) / 256), 256, 0, s>>>(fine ? M.nodes0 : M.nodes + P.nl_off[l],
+      k_mg_prolong_flat<<<(unsigned)((items + 255) / 256), 256, 0, s>>>(fine ? M.nodes0 : M.nodes + P.ns_off[l],
                                                                           items, dl, dc, M.z, cur, act);
   }
   if (fine) I.end(kcMgTransfer, q, vb * (2.0 + 1.0 / 8.0), 0);
@@ -1567,7 +1586,7 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   cudaStream_t s = I.stream;
   static const MgPlan kNoLevels;
   const MgPlan& P = M ? *M->P : kNoLevels;
-  const int nseg = 6 + 5 * P.nlev;
+  const int nseg = 6 + 6 * P.nlev;
   int e;
   if ((e = ensure(I, bCompactCnt, sizeof(int) * nseg, msg))) return e;
   if ((e = ensure(I, bTilesIc, sizeof(Tile) * std::max<int64_t>(W.nti, 1), msg))) return e;
@@ -1597,11 +1616,12 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   launch_compact(W.chunks, W.nchunks, act, cc, cnt + 4, s);
   launch_compact(W.bt, W.nbt, act, bt, cnt + 5, s);
   for (int l = 0; l < P.nlev; ++l) {
-    launch_compact(M->tiles + P.sm_off[l], P.sm_n[l], act, mt + P.sm_off[l], cnt + 6 + 5 * l, s);
-    launch_compact(M->tiles + P.in_off[l], P.in_n[l], act, mt + P.in_off[l], cnt + 7 + 5 * l, s);
-    launch_compact(M->lists + P.list_off[l], P.list_n[l], act, ml + P.list_off[l], cnt + 8 + 5 * l, s);
-    launch_compact(M->nodes + P.nl_off[l], P.nl_n[l], act, mn + P.nl_off[l], cnt + 9 + 5 * l, s);
-    launch_compact(M->tiles + P.sw_off[l], P.sw_n[l], act, mt + P.sw_off[l], cnt + 10 + 5 * l, s);
+    launch_compact(M->tiles + P.sm_off[l], P.sm_n[l], act, mt + P.sm_off[l], cnt + 6 + 6 * l, s);
+    launch_compact(M->tiles + P.in_off[l], P.in_n[l], act, mt + P.in_off[l], cnt + 7 + 6 * l, s);
+    launch_compact(M->lists + P.list_off[l], P.list_n[l], act, ml + P.list_off[l], cnt + 8 + 6 * l, s);
+    launch_compact(M->nodes + P.nl_off[l], P.nl_n[l], act, mn + P.nl_off[l], cnt + 9 + 6 * l, s);
+    launch_compact(M->tiles + P.sw_off[l], P.sw_n[l], act, mt + P.sw_off[l], cnt + 10 + 6 * l, s);
+    launch_compact(M->nodes + P.ns_off[l], P.ns_n[l], act, mn + P.ns_off[l], cnt + 11 + 6 * l, s);
   }
   launches += nseg;
   if ((e = launch_check(msg))) return e;
@@ -1622,11 +1642,12 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
     Mc->lists = ml;
     Mc->nodes = mn;
     for (int l = 0; l < P.nlev; ++l) {
-      Pc->sm_n[l] = h[6 + 5 * l];
-      Pc->in_n[l] = h[7 + 5 * l];
-      Pc->list_n[l] = h[8 + 5 * l];
-      Pc->nl_n[l] = h[9 + 5 * l];
-      Pc->sw_n[l] = h[10 + 5 * l];
+      Pc->sm_n[l] = h[6 + 6 * l];
+      Pc->in_n[l] = h[7 + 6 * l];
+      Pc->list_n[l] = h[8 + 6 * l];
+      Pc->nl_n[l] = h[9 + 6 * l];
+      Pc->sw_n[l] = h[10 + 6 * l];
+      Pc->ns_n[l] = h[11 + 6 * l];
     }
   }
   return DTC_OK;
@@ -1728,6 +1749,7 @@ int run_cg_mg(DeviceSolver::Impl& I, int ndom, int nactive, const Work& W, const
   Pc.sw_off = M.P->sw_off; Pc.sw_n = M.P->sw_n; Pc.sw_len = M.P->sw_len;
   Pc.list_off = M.P->list_off; Pc.list_n = M.P->list_n;
   Pc.nl_off = M.P->nl_off; Pc.nl_n = M.P->nl_n;
+  Pc.ns_off = M.P->ns_off; Pc.ns_n = M.P->ns_n; Pc.tail = M.P->tail;
   MgDev Mc = M;
   Mc.P = &Pc;
   int64_t listed = ndom;   // domains the current lists were compacted to
@@ -2164,7 +2186,10 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
     voxel_stiffness(8, nu, kh);
     hadamard_entries(kh, wh);
     for (int i = 0; i < kWhNum; ++i) wh32[i] = make_float2((float)wh[i], (float)wh[i]);
+    float kh32[576];
+    for (int i = 0; i < 576; ++i) kh32[i] = (float)kh[i];
     DTC_CUDA(cudaMemcpyToSymbolAsync(c_khat64, kh, sizeof(kh), 0, cudaMemcpyHostToDevice, s));
+    DTC_CUDA(cudaMemcpyToSymbolAsync(c_kh32, kh32, sizeof(kh32), 0, cudaMemcpyHostToDevice, s));
     DTC_CUDA(cudaMemcpyToSymbolAsync(c_wh64, wh, sizeof(wh), 0, cudaMemcpyHostToDevice, s));
     DTC_CUDA(cudaMemcpyToSymbolAsync(c_wh32, wh32, sizeof(wh32), 0, cudaMemcpyHostToDevice, s));
     if (int e = upload_tc_operand(kh, s, msg)) return e;

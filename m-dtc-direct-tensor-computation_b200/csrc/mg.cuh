@@ -26,7 +26,8 @@
 //   (level l+1: recurse, or z_{l+1} = K^-1 b)     ...  / k_mg_coarse
 //   t_l += P z_{l+1}                              k_mg_prolong_flat
 //   z_l = t_l + omega D_l^-1 (b_l - K_l t_l)      k_sweep<kSwPost>
-// Levels >= 2 apply the smoothing step twice before and twice after the coarse correction.
+// Levels >= 2 apply the smoothing step twice before and twice after the coarse correction.  In small batches
+// k_mg_tail does all of this for the last two levels of a domain.
 #pragma once
 
 namespace dtc {
@@ -270,6 +271,186 @@ __global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarse(const int* __res
   float* zp = z + vec_index(node_index(D, x + 1, y + 1, zc + 1), c, lc0);
   *reinterpret_cast<float4*>(zp) = make_float4(s[0], s[1], s[2], s[3]);
   *reinterpret_cast<float4*>(zp + 4) = make_float4(s[4], s[5], s[6], s[7]);
+}
+
+// The last two levels of the domains whose coarsest level the list holds (level l of at most 8^3 voxels, level
+// l + 1 of at most 4^3): pre-smoothing, residual, restriction, dense solve, prolongation and post-smoothing of 4
+// load cases of one domain in one CTA, in shared memory.  As kernels of their own these steps are 6 (8 where the
+// level smooths twice) launches of a few microseconds, each a serial chain over a grid too small for the card.
+// A thread applies K to one node and load case from the differences to its 26 neighbours, which keeps
+// rigid translations exact null vectors.  Bound by shared-memory reads (81 a node and load case) and the
+// latency between its 7 (11) barriers.  One domain of 16^3: coarse levels 1.34 -> 0.71 ms of a solve, the solve
+// 4.7 -> 3.6 ms; 16 domains of 32^3 with 60 load cases 32 -> 23 ms, the solve 148 -> 115.
+constexpr int kTailThreads = 512, kTailLc = 4, kTailN = 9, kTailIn = 7;   // nodes per edge, interior ones
+constexpr int kTailVec = kTailN * kTailN * kTailN * 3 * kTailLc;
+constexpr int kTailItems = kTailIn * kTailIn * kTailIn * kTailLc;
+constexpr int kTailCoarse = 5 * 5 * 5 * 3 * kTailLc;
+constexpr int kTailFloats = 2 * kTailVec + 3 * kTailItems + 6 * kTailItems / kTailLc + 512 + kMgDenseN * kMgDenseN +
+                            kMgDenseN * kTailLc + kTailCoarse;
+constexpr int kTailSmem = 4 * kTailFloats + kTailItems / kTailLc;
+
+// sum over the 8 voxels around a node of s_v Khat (u - u(node)); u: the node's load case in the staged
+// vector, sv: its voxel on the low sides (stride 8)
+__device__ __forceinline__ void tail_apply(const float* u, const float* sv, float (&r)[3]) {
+  constexpr int X = 3 * kTailLc, Y = kTailN * X, Z = kTailN * Y;
+  float d[27][3];
+#pragma unroll
+  for (int n = 0; n < 27; ++n)
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      d[n][c] = u[(n % 3 - 1) * X + (n / 3 % 3 - 1) * Y + (n / 9 - 1) * Z + c * kTailLc];
+#pragma unroll
+  for (int n = 0; n < 27; ++n)
+    if (n != 13)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d[n][c] -= d[13][c];
+  r[0] = r[1] = r[2] = 0.f;
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const int vx = v & 1, vy = v >> 1 & 1, vz = v >> 2;   // 0: the voxel on the low side
+    const int a = corner_local(1 - vx, 1 - vy, 1 - vz);
+    float k[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int qx = q & 1, qy = q >> 1 & 1, qz = q >> 2, e = corner_local(qx, qy, qz);
+      const int n = (vx + qx) + 3 * (vy + qy) + 9 * (vz + qz);
+      if (e == a) continue;
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) k[i] = fmaf(c_kh32[3 * a + i + 24 * (3 * e + j)], d[n][j], k[i]);
+    }
+    const float s = sv[vx + 8 * vy + 64 * vz];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) r[i] = fmaf(s, k[i], r[i]);
+  }
+}
+
+__global__ void __launch_bounds__(kTailThreads, 1)
+    k_mg_tail(const int* __restrict__ list, const DomDev* __restrict__ doms_f, const DomDev* __restrict__ doms_c,
+              const float* __restrict__ svox, const uint8_t* __restrict__ flags, const float* __restrict__ binv,
+              const float* __restrict__ minv, const float* __restrict__ b, float* __restrict__ z, float omega,
+              int steps, const int* __restrict__ dom_active) {
+  extern __shared__ __align__(16) unsigned char tail_smem[];
+  constexpr int kNodes = kTailItems / kTailLc, NT = kTailThreads;
+  float* src = reinterpret_cast<float*>(tail_smem);
+  float* dst = src + kTailVec;
+  float* sb = dst + kTailVec;                       // b, [item][3]
+  float* sd = sb + 3 * kTailItems;                  // D^-1, [node][6]
+  float* sv = sd + 6 * kNodes;                      // voxel factors, 8^3
+  float* sm = sv + 512;                             // dense inverse
+  float* bc = sm + kMgDenseN * kMgDenseN;           // [81][4]
+  float* zc = bc + kMgDenseN * kTailLc;             // [5^3][3][4], zero on the box
+  unsigned char* on = reinterpret_cast<unsigned char*>(zc + kTailCoarse);   // the node is an unknown
+  const int dom = list[blockIdx.x / (kNLC / kTailLc)], lc0 = (int)(blockIdx.x % (kNLC / kTailLc)) * kTailLc;
+  if (dom_active && !dom_active[dom]) return;
+  const DomDev& F = doms_f[dom];
+  const DomDev& C = doms_c[dom];
+  const int tid = threadIdx.x, n0 = F.n[0], n1 = F.n[1], n2 = F.n[2];
+  const int64_t node_off = F.node_off;
+  const float scale = (float)F.scale;
+  auto at = [](int x, int y, int zz) { return (x + kTailN * (y + kTailN * zz)) * 3 * kTailLc; };
+  for (int i = tid; i < 2 * kTailVec; i += NT) src[i] = 0.f;
+  for (int i = tid; i < kTailCoarse; i += NT) zc[i] = 0.f;
+  for (int i = tid; i < 512; i += NT) {
+    const int x = i % 8, y = i / 8 % 8, zz = i / 64;
+    sv[i] = x < n0 - 1 && y < n1 - 1 && zz < n2 - 1
+                ? scale * __ldg(svox + F.vox_off + x + (int64_t)(n0 - 1) * (y + (int64_t)(n1 - 1) * zz)) : 0.f;
+  }
+  for (int i = tid; i < kMgDenseN * kMgDenseN; i += NT) sm[i] = __ldg(minv + (int64_t)dom * kMgDenseN * kMgDenseN + i);
+  for (int i = tid; i < kNodes; i += NT) {
+    const int x = i % kTailIn + 1, y = i / kTailIn % kTailIn + 1, zz = i / (kTailIn * kTailIn) + 1;
+    const int64_t n = node_off + x + (int64_t)n0 * (y + (int64_t)n1 * zz);
+    const bool use = x <= n0 - 2 && y <= n1 - 2 && zz <= n2 - 2 && (flags[n] & kNodeActive);
+    on[i] = use;
+    if (use)
+      for (int q = 0; q < 6; ++q) sd[6 * i + q] = omega * __ldg(binv + 6 * n + q);
+  }
+  __syncthreads();
+  // the thread's nodes, load case tid % 4; f(index of the node, its position in a vector)
+  auto nodes = [&](auto&& f) {
+#pragma unroll 1
+    for (int i = tid; i < kTailItems; i += NT) {
+      const int n = i / kTailLc;
+      if (!on[n]) continue;
+      const int x = n % kTailIn + 1, y = n / kTailIn % kTailIn + 1, zz = n / (kTailIn * kTailIn) + 1;
+      f(n, i, x, y, zz, at(x, y, zz) + tid % kTailLc);
+    }
+  };
+  auto smooth = [&](int n, const float (&r)[3], float (&v)[3]) {
+    const float* q = sd + 6 * n;
+    v[0] = q[0] * r[0] + q[3] * r[1] + q[4] * r[2];
+    v[1] = q[3] * r[0] + q[1] * r[1] + q[5] * r[2];
+    v[2] = q[4] * r[0] + q[5] * r[1] + q[2] * r[2];
+  };
+  nodes([&](int n, int i, int x, int y, int zz, int k) {
+    const int64_t g = vec_index(node_off + x + (int64_t)n0 * (y + (int64_t)n1 * zz), 0, lc0 + tid % kTailLc);
+    float r[3], v[3];
+    for (int c = 0; c < 3; ++c) sb[3 * i + c] = r[c] = __ldg(b + g + c * kNLC);
+    smooth(n, r, v);
+    for (int c = 0; c < 3; ++c) src[k + c * kTailLc] = v[c];
+  });
+  __syncthreads();
+  const int turn = steps / 2 - 1;   // the step that leaves the residual for the coarse level
+#pragma unroll 1
+  for (int step = 0; step < steps; ++step) {
+    nodes([&](int n, int i, int x, int y, int zz, int k) {
+      float r[3], v[3];
+      tail_apply(src + k, sv + (x - 1) + 8 * (y - 1) + 64 * (zz - 1), r);
+      for (int c = 0; c < 3; ++c) r[c] = sb[3 * i + c] - r[c];
+      if (step == turn) {
+        for (int c = 0; c < 3; ++c) dst[k + c * kTailLc] = r[c];
+        return;
+      }
+      smooth(n, r, v);
+      for (int c = 0; c < 3; ++c) v[c] += src[k + c * kTailLc];
+      if (step < steps - 1) {
+        for (int c = 0; c < 3; ++c) dst[k + c * kTailLc] = v[c];
+      } else {
+        const int64_t g = vec_index(node_off + x + (int64_t)n0 * (y + (int64_t)n1 * zz), 0, lc0 + tid % kTailLc);
+        for (int c = 0; c < 3; ++c) z[g + c * kNLC] = v[c];
+      }
+    });
+    __syncthreads();
+    if (step != turn) {
+      float* q = src;
+      src = dst;
+      dst = q;
+      continue;
+    }
+    // full weighting, the dense solve on at most 27 nodes, trilinear interpolation
+    const int item = tid, lc = item % kTailLc, dof = item / kTailLc, cn = dof / 3, c = dof % 3;
+    const int cx = cn % 3 + 1, cy = cn / 3 % 3 + 1, cz = cn / 9 + 1;
+    if (dof < kMgDenseN) {
+      float s = 0.f;
+#pragma unroll
+      for (int q = 0; q < 27; ++q) {
+        const int dx = q % 3 - 1, dy = q / 3 % 3 - 1, dz = q / 9 - 1;
+        const float w = (dx ? 0.5f : 1.f) * (dy ? 0.5f : 1.f) * (dz ? 0.5f : 1.f);
+        s = fmaf(w, dst[at(2 * cx + dx, 2 * cy + dy, 2 * cz + dz) + c * kTailLc + lc], s);
+      }
+      bc[item] = cx <= C.n[0] - 2 && cy <= C.n[1] - 2 && cz <= C.n[2] - 2 ? s : 0.f;
+    }
+    __syncthreads();
+    if (dof < kMgDenseN && cx <= C.n[0] - 2 && cy <= C.n[1] - 2 && cz <= C.n[2] - 2) {
+      float s = 0.f;
+#pragma unroll 9
+      for (int k = 0; k < kMgDenseN; ++k) s = fmaf(sm[k * kMgDenseN + dof], bc[k * kTailLc + lc], s);
+      zc[((cx + 5 * (cy + 5 * cz)) * 3 + c) * kTailLc + lc] = s;
+    }
+    __syncthreads();
+    nodes([&](int, int, int x, int y, int zz, int k) {
+      float s[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int px = (x + (q & 1)) >> 1, py = (y + (q >> 1 & 1)) >> 1, pz = (zz + (q >> 2)) >> 1;
+        for (int c2 = 0; c2 < 3; ++c2)
+          s[c2] = fmaf(0.125f, zc[((px + 5 * (py + 5 * pz)) * 3 + c2) * kTailLc + tid % kTailLc], s[c2]);
+      }
+      for (int c2 = 0; c2 < 3; ++c2) src[k + c2 * kTailLc] += s[c2];
+    });
+    __syncthreads();
+  }
 }
 
 }  // namespace dtc
