@@ -33,10 +33,9 @@ LADDER = [float(f"{m}e-{k}") for k in range(3, 10) for m in (5, 3, 2, 1)][3:]
 # the host-only reference arm cannot calibrate itself
 REF_RTOL = 5e-7
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic byte of the fine
-# sweeps, measured on 16 domains of 32^3 (profiles/k_matvec_k_mg_matvec_f32_16x32cubed.md: the
-# voxel-outer sweeps at their tuned 6 or 8 CTAs per SM; below 1 where part of the input vector
-# was still in L2)
-DRAM_PER_ALGORITHMIC_BYTE = {"matvec_f32": 0.46, "mg_residual_f32": 0.97, "mg_postsmooth_f32": 1.01}
+# sweeps, measured on 16 domains of 32^3 (profiles/k_sweep_f32_16x32cubed.md; below 1 where part of the input
+# vector was still in L2)
+DRAM_PER_ALGORITHMIC_BYTE = {"matvec_f32": 0.44, "mg_residual_f32": 0.93, "mg_postsmooth_f32": 0.99}
 # FP32 SIMT FMA peak, nominal: 148 SMs x 128 lanes x 2 flop x 1.965 GHz (the sweeps run on the
 # FMA pipe, not on tensor cores; the measured peaks cover HBM and bf16 tensor only)
 FP32_NOMINAL_TFLOPS = 74.4
@@ -619,9 +618,7 @@ def main():
         us = {k[len("autotune_"):]: 1e3 * v["ms_total"] / max(v["launches"], 1) for k, v in tune.items()}
         autotune = {"timed_us_per_launch": us,
                     "pick": "tensor" if us.get("tc_sweep", 1e30) < us.get("simt_sweep", 1e30) else "simt",
-                    "note": "simt_sweep / tc_sweep: fine post-smoothing; *_6cta / *_8cta: the SIMT residual, "
-                            "post-smoothing and CG-application sweeps at 6 or 8 CTAs per SM; f64_*: the FP64 "
-                            "sweep at 4 or 6 CTAs per SM"}
+                    "note": "simt_sweep / tc_sweep: the fine post-smoothing (HEX08) or operator (HEX20)"}
     top = max((k for k in ks if ks[k]["bytes_per_launch"] > 0), key=lambda k: ks[k]["ms_total"])
     kt = ks[top]
     t_launch = kt["ms_total"] / kt["launches"] / 1e3
@@ -650,7 +647,7 @@ def main():
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": traffic, "peak_source": src,
                              "traffic_source": (f"ncu dram bytes / algorithmic bytes = {ratio} on the 16x32^3 case "
-                                                "(profiles/k_matvec_k_mg_matvec_f32_16x32cubed.md), scaled to this "
+                                                "(profiles/k_sweep_f32_16x32cubed.md), scaled to this "
                                                 "launch" if ratio else None),
                              "kernel": top, "avg_launch_us": t_launch * 1e6,
                              "flops_per_launch": kt["flops_per_launch"],

@@ -1359,7 +1359,7 @@ struct MgDev {
   const int64_t* nodes;  // levels >= 1: active interior nodes (segments nl_off / nl_n of the plan)
   float *b, *t, *z;      // levels >= 1
   float *t0, *z0;        // fine level
-  int nen0;              // element of the fine level; HEX20 applies K with the brick kernel
+  int nen0;              // element of the fine level; HEX20 applies K on columns or bricks
   const Tile* bricks0;   // fine-level interior columns (HEX20) and, for the tensor cores, bricks
   int64_t nbricks0;
   int layers0;           // voxel layers of a column

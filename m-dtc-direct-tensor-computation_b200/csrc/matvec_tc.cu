@@ -4,7 +4,7 @@
 // application, the multigrid residual and the post-smoothing -- with the 24 x 24 voxel
 // contraction as tcgen05.mma kind::tf32, A (voxel DOFs x load cases) in tensor memory, B (the
 // unit voxel stiffness) in shared memory.  HEX20 (k_ebe_tc): the 60 x 60 element contraction
-// of the brick kernel, A and B in shared memory.  Both split FP32 operands into tf32 hi + lo
+// on voxel bricks, A and B in shared memory.  Both split FP32 operands into tf32 hi + lo
 // parts (three products) for FP32-level accuracy and bound every wait.
 #include <cuda_runtime.h>
 

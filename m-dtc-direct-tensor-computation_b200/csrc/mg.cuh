@@ -39,7 +39,7 @@ enum { kMgRes = 0, kMgPost = 1 };
 constexpr int kListShift = 40;
 constexpr int64_t kListNodeMask = (int64_t(1) << kListShift) - 1;
 
-// Node-local second half of the residual / smoother when K t was applied by the brick kernel
+// Node-local second half of the residual / smoother when K t was applied on its own
 // (HEX20 fine level), z holding -K t on entry:
 //   kMgRes : z = b + z
 //   kMgPost: z = t + omega D^-1 (b + z)
