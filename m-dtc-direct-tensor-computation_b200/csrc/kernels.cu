@@ -386,6 +386,12 @@ __global__ void __launch_bounds__(kCgThreads) k_update(const Chunk* __restrict__
   }
 }
 
+}  // namespace dtc
+
+#include "tile_cg.cuh"
+
+namespace dtc {
+
 // z = M^-1 r; acc_zz += z.z ; acc_zr += z.r (start of a solve)
 template <typename T, bool BLOCK>
 __global__ void __launch_bounds__(kThreads) k_initial_dots(const Tile* __restrict__ tiles,
@@ -807,7 +813,7 @@ enum Buf { bDoms, bTilesI, bTilesA, bSvox, bFlags, bDinv64, bDinv32, bX, bR64, b
            bMgDoms, bMgTiles, bMgSvox, bMgFlags, bMgDinv64, bMgDinv32, bMgBinv32, bMgB, bMgT, bMgZ, bMgMinv, bMgList,
            bAdjG, bAdjV, bAdjBlk, bAdjGrad, bAdjDoms, bAdjX, bAdjSvox, bKe20tc, bBricksTc, bBricksTcC, bNodesI,
            bTilesIc, bNodesIc, bBricksIc, bMgTilesC, bMgListC, bCompactCnt, bMgNodes, bMgNodesC, bXkeep, bTilesW, bTilesWa,
-           bTilesWc, bChunks, bChunksC, bNChunk, bBlkSt, bBlkCf, bGram, bGramDone, bNumBufs };
+           bTilesWc, bTilesF, bTilesFc, bChunks, bChunksC, bNChunk, bBlkSt, bBlkCf, bGram, bGramDone, bNumBufs };
 static_assert(bNumBufs <= 80, "buffer table");
 static_assert(bSvox == 3, "DeviceSolver::Impl::svox() reads bufs[3]");
 
@@ -919,6 +925,9 @@ struct Work {
   int64_t nbt = 0;
   const Chunk* chunks = nullptr;   // the node list in pieces of one domain (CG vector kernels)
   int64_t nchunks = 0;
+  bool tile_walk = false;          // plain FP64 CG on node tiles (tile_cg.cuh), and the operator's tiles
+  const Tile* tf = nullptr;
+  int64_t ntf = 0;
 };
 
 // One HEX08 sweep over nt tiles of len nodes in x.
@@ -929,6 +938,14 @@ void launch_sweep(int64_t nt, int len, cudaStream_t s, const Tile* tiles, const 
   if (nt <= 0) return;
   const unsigned g = (unsigned)(nt * (kNLC / (4 * Lane<T>::kCols)));
   k_sweep<T, ALL, MODE><<<g, kSweepThreads, kSweepSmem, s>>>(tiles, len, dd, svox, u, y, scale, binv, b, omega, acc, act);
+}
+
+// The HEX08 operator over the interior nodes on node tiles (tile_cg.cuh).
+template <bool DOT>
+void launch_tile_matvec(const Work& W, const DomDev* dd, const float* svox, const double* u, double* y, double scale,
+                        double* acc, const int* act, int bnd_only, cudaStream_t s) {
+  if (W.ntf <= 0) return;
+  k_tile_matvec<DOT><<<(unsigned)(3 * W.ntf), kThreads, 0, s>>>(W.tf, dd, svox, u, y, scale, acc, act, bnd_only);
 }
 
 template <typename T, bool ALL, int MODE>
@@ -1586,11 +1603,12 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   cudaStream_t s = I.stream;
   static const MgPlan kNoLevels;
   const MgPlan& P = M ? *M->P : kNoLevels;
-  const int nseg = 6 + 6 * P.nlev;
+  const int nseg = 7 + 6 * P.nlev;
   int e;
   if ((e = ensure(I, bCompactCnt, sizeof(int) * nseg, msg))) return e;
   if ((e = ensure(I, bTilesIc, sizeof(Tile) * std::max<int64_t>(W.nti, 1), msg))) return e;
   if ((e = ensure(I, bTilesWc, sizeof(Tile) * std::max<int64_t>(W.ntw, 1), msg))) return e;
+  if ((e = ensure(I, bTilesFc, sizeof(Tile) * std::max<int64_t>(W.ntf, 1), msg))) return e;
   if ((e = ensure(I, bNodesIc, sizeof(int64_t) * std::max<int64_t>(W.nnodes, 1), msg))) return e;
   if ((e = ensure(I, bBricksIc, sizeof(Tile) * std::max<int64_t>(W.nbi, 1), msg))) return e;
   if ((e = ensure(I, bBricksTcC, sizeof(Tile) * std::max<int64_t>(W.nbt, 1), msg))) return e;
@@ -1602,6 +1620,7 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   DTC_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * nseg, s));
   Tile* tc = B<Tile>(I, bTilesIc);
   Tile* wc = B<Tile>(I, bTilesWc);
+  Tile* fc = B<Tile>(I, bTilesFc);
   int64_t* nc = B<int64_t>(I, bNodesIc);
   Tile* bc = B<Tile>(I, bBricksIc);
   Tile* bt = B<Tile>(I, bBricksTcC);
@@ -1615,13 +1634,14 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   launch_compact(W.tw, W.ntw, act, wc, cnt + 3, s);
   launch_compact(W.chunks, W.nchunks, act, cc, cnt + 4, s);
   launch_compact(W.bt, W.nbt, act, bt, cnt + 5, s);
+  launch_compact(W.tf, W.ntf, act, fc, cnt + 6, s);
   for (int l = 0; l < P.nlev; ++l) {
-    launch_compact(M->tiles + P.sm_off[l], P.sm_n[l], act, mt + P.sm_off[l], cnt + 6 + 6 * l, s);
-    launch_compact(M->tiles + P.in_off[l], P.in_n[l], act, mt + P.in_off[l], cnt + 7 + 6 * l, s);
-    launch_compact(M->lists + P.list_off[l], P.list_n[l], act, ml + P.list_off[l], cnt + 8 + 6 * l, s);
-    launch_compact(M->nodes + P.nl_off[l], P.nl_n[l], act, mn + P.nl_off[l], cnt + 9 + 6 * l, s);
-    launch_compact(M->tiles + P.sw_off[l], P.sw_n[l], act, mt + P.sw_off[l], cnt + 10 + 6 * l, s);
-    launch_compact(M->nodes + P.ns_off[l], P.ns_n[l], act, mn + P.ns_off[l], cnt + 11 + 6 * l, s);
+    launch_compact(M->tiles + P.sm_off[l], P.sm_n[l], act, mt + P.sm_off[l], cnt + 7 + 6 * l, s);
+    launch_compact(M->tiles + P.in_off[l], P.in_n[l], act, mt + P.in_off[l], cnt + 8 + 6 * l, s);
+    launch_compact(M->lists + P.list_off[l], P.list_n[l], act, ml + P.list_off[l], cnt + 9 + 6 * l, s);
+    launch_compact(M->nodes + P.nl_off[l], P.nl_n[l], act, mn + P.nl_off[l], cnt + 10 + 6 * l, s);
+    launch_compact(M->tiles + P.sw_off[l], P.sw_n[l], act, mt + P.sw_off[l], cnt + 11 + 6 * l, s);
+    launch_compact(M->nodes + P.ns_off[l], P.ns_n[l], act, mn + P.ns_off[l], cnt + 12 + 6 * l, s);
   }
   launches += nseg;
   if ((e = launch_check(msg))) return e;
@@ -1634,6 +1654,7 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   Wc.tw = wc; Wc.ntw = h[3];
   Wc.chunks = cc; Wc.nchunks = h[4];
   Wc.bt = bt; Wc.nbt = h[5];
+  Wc.tf = fc; Wc.ntf = h[6];
   if (M) {
     Mc->bricks0 = bc; Mc->nbricks0 = h[2];
     Mc->tcbricks0 = bt; Mc->ntcbricks0 = h[5];
@@ -1642,12 +1663,12 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
     Mc->lists = ml;
     Mc->nodes = mn;
     for (int l = 0; l < P.nlev; ++l) {
-      Pc->sm_n[l] = h[6 + 6 * l];
-      Pc->in_n[l] = h[7 + 6 * l];
-      Pc->list_n[l] = h[8 + 6 * l];
-      Pc->nl_n[l] = h[9 + 6 * l];
-      Pc->sw_n[l] = h[10 + 6 * l];
-      Pc->ns_n[l] = h[11 + 6 * l];
+      Pc->sm_n[l] = h[7 + 6 * l];
+      Pc->in_n[l] = h[8 + 6 * l];
+      Pc->list_n[l] = h[9 + 6 * l];
+      Pc->nl_n[l] = h[10 + 6 * l];
+      Pc->sw_n[l] = h[11 + 6 * l];
+      Pc->ns_n[l] = h[12 + 6 * l];
     }
   }
   return DTC_OK;
@@ -1660,6 +1681,8 @@ int run_cg(DeviceSolver::Impl& I, int ndom, const Work& W, T* x, T* r, T* p, T* 
   // work lists: the full ones until half the domains have converged, then compacted copies
   Work Wc = W;
   int64_t listed = ndom;
+  constexpr bool kTiles = sizeof(T) == 8 && !BLOCK && NEN == 8;
+  const bool walk = kTiles && W.tile_walk;
   const DomDev* dd = B<DomDev>(I, bDoms);
   const uint8_t* fl = B<uint8_t>(I, bFlags);
   ColState* st = B<ColState>(I, bSt);
@@ -1689,7 +1712,21 @@ int run_cg(DeviceSolver::Impl& I, int ndom, const Work& W, T* x, T* r, T* p, T* 
     const unsigned gb = (unsigned)Wc.nchunks;
     auto body = [&](int64_t& nl) {
       for (int k = 0; k < chunk; ++k) {
-        if (nti > 0) {
+        if (nti > 0 && walk) {
+          if constexpr (kTiles) {
+            const unsigned gi = (unsigned)(3 * nti);
+            int q = I.begin(0);
+            k_tile_direction<<<gi, kThreads, 0, s>>>(ti, dd, fl, dinv, r, p, st, act);
+            I.end(kcDirection64, q, 3 * vb, 0);
+            q = I.begin(0);
+            launch_tile_matvec<true>(Wc, dd, I.svox(), p, w, 1.0, pw, act, 0, s);
+            I.end(kcMatvec64, q, mb, mf);
+            q = I.begin(0);
+            k_tile_update<<<gi, kThreads, 0, s>>>(ti, dd, fl, dinv, x, r, p, w, st, pw, zz, zr, act);
+            I.end(kcUpdate64, q, 6 * vb, 0);
+            nl += 3;
+          }
+        } else if (nti > 0) {
           int q = I.begin(0);
           k_direction<T, BLOCK><<<gb, kCgThreads, 0, s>>>(Wc.chunks, W.nodes, dinv, r, p, st, act);
           I.end(f32 ? kcDirection32 : kcDirection64, q, 3 * vb, 0);
@@ -1954,6 +1991,9 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
   return DTC_OK;
 }
 
+// Whether a solve runs the plain FP64 CG in the fixed summation order of the node tiles (HEX08).
+inline bool tile_walk(const dtc_options& opt) { return opt.precision != DTC_PREC_MIXED && opt.rtol > kTightRtol; }
+
 struct HostBatch {
   int nen = 0;
   std::vector<int64_t> tidx;   // tasks solved in this pass
@@ -1961,6 +2001,7 @@ struct HostBatch {
   std::vector<Tile> tiles_i, tiles_a, bricks_i, bricks_a, bricks_t;
   int layers = 1;              // voxel layers of a HEX20 column
   std::vector<Tile> tiles_w, tiles_wa;   // sweep tiles (HEX08) over the interior / all nodes
+  std::vector<Tile> tiles_f;             // operator tiles of the plain FP64 CG on node tiles (else empty)
   int sweep_len = kSweepX;               // their nodes in x
   std::vector<int64_t> nodes_i;
   std::vector<Chunk> chunks;   // nodes_i cut into pieces of one domain (CG vector kernels)
@@ -2007,11 +2048,12 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
   if (NEN == 20) hb.layers = hex20_layers(grids);
   const bool bricks_tc = opt.precision == DTC_PREC_MIXED && opt.mixed_matvec != 0;
   const int len = hb.sweep_len;
+  const bool walk = NEN == 8 && tile_walk(opt);
   svox.assign((size_t)vox_total, 0.f);
   // per domain: voxel factors, node activity and work lists (host threads)
   struct Packed {
     DomDev D;
-    std::vector<Tile> ti, ta, bi, ba, bt, tw, twa;
+    std::vector<Tile> ti, ta, bi, ba, bt, tw, twa, tf;
     std::vector<int64_t> ni;
     double vec = 0, mv = 0, fl = 0;
   };
@@ -2100,6 +2142,12 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
             if (any_active(x0, y0, z0, len, kSweepY, kSweepZ, 0, nx - 1, ny - 1, nz - 1))
               out.twa.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
     }
+    if (walk)
+      for (int z0 = 1; z0 <= nz - 2; z0 += kTileZ)
+        for (int y0 = 1; y0 <= ny - 2; y0 += kTileY)
+          for (int x0 = 1; x0 <= nx - 2; x0 += kSweepX)
+            if (any_active(x0, y0, z0, kSweepX, kTileY, kTileZ, 1, nx - 2, ny - 2, nz - 2))
+              out.tf.push_back(Tile{dom, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
     for (int z0 = 0; z0 <= nz - 1; z0 += kTileZ)
       for (int y0 = 0; y0 <= ny - 1; y0 += kTileY)
         for (int x0 = 0; x0 <= nx - 1; x0 += kTileX)
@@ -2138,6 +2186,7 @@ int prepare_nen(std::vector<DomainTask>& tasks, const dtc_options& opt, double n
     tiles_a.insert(tiles_a.end(), q.ta.begin(), q.ta.end());
     hb.tiles_w.insert(hb.tiles_w.end(), q.tw.begin(), q.tw.end());
     hb.tiles_wa.insert(hb.tiles_wa.end(), q.twa.begin(), q.twa.end());
+    hb.tiles_f.insert(hb.tiles_f.end(), q.tf.begin(), q.tf.end());
     bricks_i.insert(bricks_i.end(), q.bi.begin(), q.bi.end());
     bricks_a.insert(bricks_a.end(), q.ba.begin(), q.ba.end());
     hb.bricks_t.insert(hb.bricks_t.end(), q.bt.begin(), q.bt.end());
@@ -2246,6 +2295,8 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   if ((e = ensure(I, bTilesW, sizeof(Tile) * std::max<int64_t>(ntw, 1), msg))) return e;
   const int64_t ntwa = (int64_t)hb.tiles_wa.size();
   if ((e = ensure(I, bTilesWa, sizeof(Tile) * std::max<int64_t>(ntwa, 1), msg))) return e;
+  const int64_t ntf = (int64_t)hb.tiles_f.size();
+  if ((e = ensure(I, bTilesF, sizeof(Tile) * std::max<int64_t>(ntf, 1), msg))) return e;
   if ((e = ensure(I, bBricksI, sizeof(Tile) * std::max<int64_t>(nbi, 1), msg))) return e;
   const int64_t nbt = (int64_t)hb.bricks_t.size();
   if ((e = ensure(I, bBricksTc, sizeof(Tile) * std::max<int64_t>(nbt, 1), msg))) return e;
@@ -2299,6 +2350,8 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
     DTC_CUDA(cudaMemcpyAsync(I.bufs[bTilesW], hb.tiles_w.data(), sizeof(Tile) * ntw, cudaMemcpyHostToDevice, s));
   if (ntwa)
     DTC_CUDA(cudaMemcpyAsync(I.bufs[bTilesWa], hb.tiles_wa.data(), sizeof(Tile) * ntwa, cudaMemcpyHostToDevice, s));
+  if (ntf)
+    DTC_CUDA(cudaMemcpyAsync(I.bufs[bTilesF], hb.tiles_f.data(), sizeof(Tile) * ntf, cudaMemcpyHostToDevice, s));
   if (nbi) DTC_CUDA(cudaMemcpyAsync(I.bufs[bBricksI], bricks_i.data(), sizeof(Tile) * nbi, cudaMemcpyHostToDevice, s));
   if ((e = ensure(I, bNodesI, sizeof(int64_t) * std::max<size_t>(nodes_i.size(), 1), msg))) return e;
   if (!nodes_i.empty())
@@ -2343,6 +2396,9 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   W.len = hb.sweep_len;
   W.chunks = B<Chunk>(I, bChunks);
   W.nchunks = (int64_t)hb.chunks.size();
+  W.tile_walk = NEN == 8 && tile_walk(opt);
+  W.tf = B<Tile>(I, bTilesF);
+  W.ntf = ntf;
   const DomDev* dd = B<DomDev>(I, bDoms);
   uint8_t* fl = B<uint8_t>(I, bFlags);
   double* X = B<double>(I, bX);
@@ -2500,7 +2556,8 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
       // b = -(K X)_interior with X = boundary values only (RHS of all 24 load cases, :674-951)
       DTC_CUDA(cudaMemsetAsync(I.bufs[bP64], 0, vbytes64, s));
       DTC_CUDA(cudaMemsetAsync(I.bufs[bW64], 0, vbytes64, s));
-      apply_k<double, NEN, false, false>(W, dd, I.svox(), fl, X, R64, -1.0, nullptr, nullptr, s);
+      if (W.tile_walk) launch_tile_matvec<false>(W, dd, I.svox(), X, R64, -1.0, nullptr, nullptr, 1, s);
+      else apply_k<double, NEN, false, false>(W, dd, I.svox(), fl, X, R64, -1.0, nullptr, nullptr, s);
       ++L;
       if ((e = run_cg<double, false, NEN>(I, ndom, W, X, R64, B<double>(I, bP64), B<double>(I, bW64), B<double>(I, bDinv64),
                               opt.rtol, nullptr, opt.max_it, L, msg)))
