@@ -33,13 +33,15 @@
 
 namespace dtc {
 
-__constant__ double c_khat64[576];   // unit voxel stiffness, column-major (symmetric)
-__constant__ float c_kh32[576];      // the same in FP32 (k_mg_tail)
+// Matrices and modes that depend on a solve's options are kernel arguments, which the constant bank serves: a
+// __constant__ symbol is one per device, and handles in other threads solve with other options.
+template <typename T> struct VoxelMatrix { T v[576]; };   // unit voxel stiffness, column-major (symmetric)
 // the 24 load-case columns of the current column pass of the macro modes for eps = 1e-6:
 // uu(nm,3,24) column-major, nm = 8 (macro order 1) or 20 (macro order 2); columns past the
 // last load case are zero
-__constant__ double c_uu[20 * 3 * kNLC];
-__constant__ double c_k20_64[3600];       // unit HEX20 element matrix (ring node order)
+struct MacroModes { double uu[20 * 3 * kNLC]; };
+// 3 x 3 diagonal blocks of a unit element matrix, node by node, row-major
+template <int NEN> struct NodeBlocks { double b[NEN][9]; };
 
 }  // namespace dtc
 
@@ -63,16 +65,21 @@ template <> __device__ __forceinline__ int local_node<20>(int ox, int oy, int oz
     if (ring_off(a, 0) == ox && ring_off(a, 1) == oy && ring_off(a, 2) == oz) return a;
   return -1;
 }
-template <int NEN> __device__ __forceinline__ double ke64(int i);
-template <> __device__ __forceinline__ double ke64<8>(int i) { return c_khat64[i]; }
-template <> __device__ __forceinline__ double ke64<20>(int i) { return c_k20_64[i]; }
+template <int NEN>
+NodeBlocks<NEN> node_blocks(const double* ke) {   // ke column-major
+  NodeBlocks<NEN> B;
+  for (int n = 0; n < NEN; ++n)
+    for (int a = 0; a < 3; ++a)
+      for (int b = 0; b < 3; ++b) B.b[n][3 * a + b] = ke[(3 * n + a) + 3 * NEN * (3 * n + b)];
+  return B;
+}
 
 template <int NEN>
 __global__ void __launch_bounds__(kThreads) k_node_setup(const Tile* __restrict__ tiles, const DomDev* __restrict__ doms,
                                                          const float* __restrict__ svox, uint8_t* __restrict__ flags,
                                                          double* __restrict__ dinv64, float* __restrict__ dinv32,
-                                                         float* __restrict__ binv32) {
-  constexpr int ND = 3 * NEN;
+                                                         float* __restrict__ binv32,
+                                                         const __grid_constant__ NodeBlocks<NEN> ke) {
   const Tile t = tiles[blockIdx.x];
   const DomDev D = doms[t.dom];
   const int x = t.x0 + (threadIdx.x & 7), row = threadIdx.x >> 3;
@@ -98,9 +105,9 @@ __global__ void __launch_bounds__(kThreads) k_node_setup(const Tile* __restrict_
         const int ln = local_node<NEN>(oc[0][i], oc[1][j], oc[2][k]);
         if (ln < 0) continue;
         active = true;
-        for (int a = 0; a < 3; ++a) d3[a] += (double)s * ke64<NEN>((3 * ln + a) * (ND + 1));
+        for (int a = 0; a < 3; ++a) d3[a] += (double)s * ke.b[ln][4 * a];
         for (int a = 0; a < 3; ++a)
-          for (int b = 0; b < 3; ++b) blk[a][b] += (double)s * ke64<NEN>((3 * ln + a) + ND * (3 * ln + b));
+          for (int b = 0; b < 3; ++b) blk[a][b] += (double)s * ke.b[ln][3 * a + b];
       }
   for (int a = 0; a < 3; ++a) d3[a] *= D.scale;
   const bool bnd = (x == 0 || x == D.n[0] - 1 || y == 0 || y == D.n[1] - 1 || z == 0 || z == D.n[2] - 1);
@@ -202,7 +209,8 @@ template <int NM>
 __global__ void __launch_bounds__(kThreads) k_boundary_values(const Tile* __restrict__ tiles,
                                                               const DomDev* __restrict__ doms,
                                                               const uint8_t* __restrict__ flags,
-                                                              double* __restrict__ X) {
+                                                              double* __restrict__ X,
+                                                              const __grid_constant__ MacroModes M) {
   const Tile t = tiles[blockIdx.x];
   const DomDev D = doms[t.dom];
   const int x = t.x0 + (threadIdx.x & 7), row = threadIdx.x >> 3;
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(kThreads) k_boundary_values(const Tile* __rest
   for (int c = 0; c < 3; ++c)
     for (int lc = 0; lc < kNLC; ++lc) {
       double s = 0.0;
-      for (int l = 0; l < NM; ++l) s += N[l] * c_uu[l + NM * c + 3 * NM * lc];
+      for (int l = 0; l < NM; ++l) s += N[l] * M.uu[l + NM * c + 3 * NM * lc];
       X[vec_index(n, c, lc)] = s;
     }
 }
@@ -733,9 +741,15 @@ struct DeviceSolver::Impl {
   cudaStream_t stream = nullptr;
   // persistent buffers grown on demand
   std::vector<std::pair<void**, size_t>> owned;
-  // HEX20 unit element matrix of the solve in hand, in its classes
+  // of the last solve: the unit voxel matrix (FP64, FP32), its Hadamard entries, and the HEX20 unit element matrix
+  // in its classes
+  VoxelMatrix<double> kh64 = {};
+  VoxelMatrix<float> kh32 = {};
+  Hadamard<double> wh64 = {};
+  Hadamard<float> wh32 = {};
   ClassBlocks<double> k20_64 = {};
   ClassBlocks<float> k20_32 = {};
+  TcCtl tc = {};   // tensor-core kernels: operand, waits
   void* bufs[80] = {nullptr};
   size_t caps[80] = {0};
   // what the solves of the last batch kept for the adjoint: per chunk the domains (node and
@@ -811,7 +825,7 @@ namespace {
 enum Buf { bDoms, bTilesI, bTilesA, bSvox, bFlags, bDinv64, bDinv32, bX, bR64, bP64, bW64, bR32, bX32, bP32, bW32,
            bSt, bOst, bPw, bZz, bZr, bDomAct, bCount, bFf, bTarget, bErr, bBinv32, bBricksI, bBricksA, bZ32, bT32,
            bMgDoms, bMgTiles, bMgSvox, bMgFlags, bMgDinv64, bMgDinv32, bMgBinv32, bMgB, bMgT, bMgZ, bMgMinv, bMgList,
-           bAdjG, bAdjV, bAdjBlk, bAdjGrad, bAdjDoms, bAdjX, bAdjSvox, bKe20tc, bBricksTc, bBricksTcC, bNodesI,
+           bAdjG, bAdjV, bAdjBlk, bAdjGrad, bAdjDoms, bAdjX, bAdjSvox, bKe20tc, bKhTc, bBricksTc, bBricksTcC, bNodesI,
            bTilesIc, bNodesIc, bBricksIc, bMgTilesC, bMgListC, bCompactCnt, bMgNodes, bMgNodesC, bXkeep, bTilesW, bTilesWa,
            bTilesWc, bTilesF, bTilesFc, bChunks, bChunksC, bNChunk, bBlkSt, bBlkCf, bGram, bGramDone, bNumBufs };
 static_assert(bNumBufs <= 80, "buffer table");
@@ -867,16 +881,17 @@ int DeviceSolver::init(int device, std::string& msg) {
 
 void launch_sweep_tc(int mode, const Tile* tiles, int64_t ntiles, const DomDev* doms, const float* svox,
                      const uint8_t* flags, const float* binv, const float* b, const float* u, float* y, float scale,
-                     float omega, double* acc, const int* dom_active, int* err, cudaStream_t s);
+                     float omega, double* acc, const int* dom_active, const TcCtl& ctl, cudaStream_t s);
 int allow_sweep_tc(std::string& msg);
-int upload_tc_operand(const double* khat, cudaStream_t s, std::string& msg);
-int set_tc_spin_limit(long long spins, cudaStream_t s, std::string& msg);
+size_t tc_operand_bytes();
+void build_tc_operand(const double* khat, float* img);
+long long tc_spin_limit(long long spins);
 void build_tc20_operand(const double* k20, float* img);
 size_t tc20_operand_bytes();
 int allow_ebe_tc(std::string& msg);
 void launch_ebe_tc(const Tile* bricks, int64_t nb, const DomDev* doms, const float* svox, const uint8_t* flags,
                    const float* bsplit, const float* u, float* y, double scale, double* acc_pw, const int* dom_active,
-                   int* err, cudaStream_t s);
+                   const TcCtl& ctl, cudaStream_t s);
 
 namespace {
 
@@ -913,11 +928,9 @@ struct Work {
   int64_t nti, nta, nbi, nba;
   const int64_t* nodes;  // active interior nodes, (domain << kListShift) | node
   int64_t nnodes;
-  const ClassBlocks<double>* ke64;   // HEX20 unit element matrix in its classes (host memory)
-  const ClassBlocks<float>* ke32;
   int layers;           // voxel layers of a HEX20 column
   const float* ke20tc;  // HEX20 FP32 applications on tcgen05: split matrix in the B layout, else null
-  int* err;             // mbarrier time-out flag of the tensor-core kernels
+  const DeviceSolver::Impl* I;   // matrices of the solve
   const Tile *tw = nullptr, *twa = nullptr;   // tiles of the HEX08 sweeps over the interior / all nodes
   int64_t ntw = 0, ntwa = 0;
   int len = kSweepX;               // their nodes in x
@@ -930,14 +943,21 @@ struct Work {
   int64_t ntf = 0;
 };
 
+template <typename T>
+const Hadamard<T>& hadamard(const DeviceSolver::Impl& I) {
+  if constexpr (sizeof(T) == 8) return I.wh64;
+  else return I.wh32;
+}
+
 // One HEX08 sweep over nt tiles of len nodes in x.
 template <typename T, bool ALL, int MODE>
-void launch_sweep(int64_t nt, int len, cudaStream_t s, const Tile* tiles, const DomDev* dd, const float* svox,
+void launch_sweep(int64_t nt, int len, cudaStream_t s, const DeviceSolver::Impl& I, const Tile* tiles, const DomDev* dd, const float* svox,
                   const T* u, T* y, double scale, const float* binv, const T* b, float omega, double* acc,
                   const int* act) {
   if (nt <= 0) return;
   const unsigned g = (unsigned)(nt * (kNLC / (4 * Lane<T>::kCols)));
-  k_sweep<T, ALL, MODE><<<g, kSweepThreads, kSweepSmem, s>>>(tiles, len, dd, svox, u, y, scale, binv, b, omega, acc, act);
+  k_sweep<T, ALL, MODE><<<g, kSweepThreads, kSweepSmem, s>>>(tiles, len, dd, svox, hadamard<T>(I), u, y, scale, binv, b,
+                                                              omega, acc, act);
 }
 
 // The HEX08 operator over the interior nodes on node tiles (tile_cg.cuh).
@@ -945,7 +965,7 @@ template <bool DOT>
 void launch_tile_matvec(const Work& W, const DomDev* dd, const float* svox, const double* u, double* y, double scale,
                         double* acc, const int* act, int bnd_only, cudaStream_t s) {
   if (W.ntf <= 0) return;
-  k_tile_matvec<DOT><<<(unsigned)(3 * W.ntf), kThreads, 0, s>>>(W.tf, dd, svox, u, y, scale, acc, act, bnd_only);
+  k_tile_matvec<DOT><<<(unsigned)(3 * W.ntf), kThreads, 0, s>>>(W.tf, dd, svox, W.I->kh64, u, y, scale, acc, act, bnd_only);
 }
 
 template <typename T, bool ALL, int MODE>
@@ -970,18 +990,18 @@ template <typename T, int NEN, bool ALL, bool DOT>
 void apply_k(const Work& W, const DomDev* dd, const float* svox, const uint8_t* fl, const T* u, T* y, double scale,
              double* acc, const int* act, cudaStream_t s) {
   if constexpr (NEN == 8) {
-    launch_sweep<T, ALL, DOT ? kSwApplyDot : kSwApply>(ALL ? W.ntwa : W.ntw, W.len, s, ALL ? W.twa : W.tw, dd, svox,
+    launch_sweep<T, ALL, DOT ? kSwApplyDot : kSwApply>(ALL ? W.ntwa : W.ntw, W.len, s, *W.I, ALL ? W.twa : W.tw, dd, svox,
                                                        u, y, scale, nullptr, nullptr, 0.f, acc, act);
   } else {
     if constexpr (sizeof(T) == 4 && !ALL) {
       if (W.ke20tc) {
-        launch_ebe_tc(W.bt, W.nbt, dd, svox, fl, W.ke20tc, u, y, scale, DOT ? acc : nullptr, act, W.err, s);
+        launch_ebe_tc(W.bt, W.nbt, dd, svox, fl, W.ke20tc, u, y, scale, DOT ? acc : nullptr, act, W.I->tc, s);
         return;
       }
     }
     const ClassBlocks<T>* ke;
-    if constexpr (sizeof(T) == 8) ke = W.ke64;
-    else ke = W.ke32;
+    if constexpr (sizeof(T) == 8) ke = &W.I->k20_64;
+    else ke = &W.I->k20_32;
     launch_hex20<T, ALL, DOT>(ALL ? W.ba : W.bi, ALL ? W.nba : W.nbi, W.layers, dd, svox, fl, *ke, u, y, scale, acc, act,
                               s);
   }
@@ -1384,16 +1404,15 @@ struct MgDev {
   int64_t ntcbricks0;
   const int64_t* nodes0; // fine-level active interior nodes, (domain << kListShift) | node
   int64_t nnodes0;
-  const ClassBlocks<float>* ke32;   // HEX20 unit element matrix in its classes (host memory)
-  const float* ke20tc;   // its tensor-core operand, or null (SIMT kernel)
-  int* err;
+  const float* ke20tc;   // HEX20: the tensor-core operand, or null (SIMT kernel)
 };
 
 // The HEX08 residual and post-smoothing sweeps of a level over nt sweep tiles.
 template <int MODE>
-void launch_mg_matvec(int64_t nt, int len, cudaStream_t s, const Tile* t, const DomDev* d, const float* sv,
+void launch_mg_matvec(const DeviceSolver::Impl& I, int64_t nt, int len, cudaStream_t s, const Tile* t, const DomDev* d, const float* sv,
                       const float* bi, const float* b, const float* u, float* y, float om, const int* act) {
-  launch_sweep<float, false, MODE == kMgRes ? kSwRes : kSwPost>(nt, len, s, t, d, sv, u, y, 1.0, bi, b, om, nullptr, act);
+  launch_sweep<float, false, MODE == kMgRes ? kSwRes : kSwPost>(nt, len, s, I, t, d, sv, u, y, 1.0, bi, b, om, nullptr,
+                                                                act);
 }
 
 // t_ready: the fine-level t = omega D^-1 r0 was already written (by k_blk_update)
@@ -1421,7 +1440,7 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   }
   if (!fine && P.tail && l + 1 < P.nlev && P.list_n[l + 1] > 0) {
     k_mg_tail<<<(unsigned)(kNLC / kTailLc * P.list_n[l + 1]), kTailThreads, kTailSmem, s>>>(
-        M.lists + P.list_off[l + 1], dl, M.doms + (size_t)(l + 1) * M.ndom, sv, fl, bi, M.minv, b, z, P.omega,
+        M.lists + P.list_off[l + 1], dl, M.doms + (size_t)(l + 1) * M.ndom, sv, I.kh32, fl, bi, M.minv, b, z, P.omega,
         l >= kMgTwiceFrom ? 4 : 2, act);
     ++launches;
   }
@@ -1453,24 +1472,24 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   float* cur = t;                  // the smoothed iterate
   float* rbuf = z;                 // the residual handed to the restriction
   if (twice) {
-    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, t, z, om, act);
+    launch_mg_matvec<kMgPost>(I, gw, sl, s, tsw, dl, sv, bi, b, t, z, om, act);
     ++launches;
     cur = z;
     rbuf = t;
   }
   if (fine && M.nen0 == 20) {
     if (M.ke20tc)
-      launch_ebe_tc(M.tcbricks0, M.ntcbricks0, dl, sv, fl, M.ke20tc, t, z, -1.0, nullptr, act, M.err, s);
+      launch_ebe_tc(M.tcbricks0, M.ntcbricks0, dl, sv, fl, M.ke20tc, t, z, -1.0, nullptr, act, I.tc, s);
     else
-      launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, dl, sv, fl, *M.ke32, t, z, -1.0, nullptr, act, s);
+      launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, dl, sv, fl, I.k20_32, t, z, -1.0, nullptr, act, s);
     k_mg_combine<kMgRes><<<g, kThreads, 0, s>>>(tsm, dl, fl, bi, b, t, z, om, act);
     ++launches;
   } else if (fine && I.tensor_matvec) {
-    launch_sweep_tc(kTcRes, tsm, nsm, dl, sv, fl, bi, b, cur, rbuf, 1.0f, om, nullptr, act, M.err, s);
+    launch_sweep_tc(kTcRes, tsm, nsm, dl, sv, fl, bi, b, cur, rbuf, 1.0f, om, nullptr, act, I.tc, s);
   } else if (fine) {
-    launch_mg_matvec<kMgRes>(gw, sl, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
+    launch_mg_matvec<kMgRes>(I, gw, sl, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
   } else {
-    launch_mg_matvec<kMgRes>(gw, sl, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
+    launch_mg_matvec<kMgRes>(I, gw, sl, s, tsw, dl, sv, bi, b, cur, rbuf, om, act);
   }
   if (fine) I.end(kcMgResidual, q, mb + vb, mf);          // t in, r out (mb), b in
   const DomDev* dc = M.doms + (size_t)(l + 1) * M.ndom;
@@ -1497,22 +1516,22 @@ void mg_vcycle(DeviceSolver::Impl& I, const MgDev& M, int l, const float* r0, co
   q = fine ? I.begin(0) : -1;
   if (l == 0 && M.nen0 == 20) {
     if (M.ke20tc)
-      launch_ebe_tc(M.tcbricks0, M.ntcbricks0, dl, sv, fl, M.ke20tc, t, z, -1.0, nullptr, act, M.err, s);
+      launch_ebe_tc(M.tcbricks0, M.ntcbricks0, dl, sv, fl, M.ke20tc, t, z, -1.0, nullptr, act, I.tc, s);
     else
-      launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, dl, sv, fl, *M.ke32, t, z, -1.0, nullptr, act, s);
+      launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, dl, sv, fl, I.k20_32, t, z, -1.0, nullptr, act, s);
     k_mg_combine<kMgPost><<<g, kThreads, 0, s>>>(tsm, dl, fl, bi, b, t, z, P.omega0, act);
     ++launches;
   } else if (l == 0 && I.tensor_matvec)
-    launch_sweep_tc(kTcPost, tsm, nsm, dl, sv, fl, bi, b, t, z, 1.0f, P.omega0, nullptr, act, M.err, s);
+    launch_sweep_tc(kTcPost, tsm, nsm, dl, sv, fl, bi, b, t, z, 1.0f, P.omega0, nullptr, act, I.tc, s);
   else if (l == 0)
-    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega0, act);
+    launch_mg_matvec<kMgPost>(I, gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega0, act);
   else if (twice) {
     // z holds the corrected iterate: t = z + w D^-1 (b - K z), then z = t + w D^-1 (b - K t)
-    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, z, t, P.omega, act);
-    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
+    launch_mg_matvec<kMgPost>(I, gw, sl, s, tsw, dl, sv, bi, b, z, t, P.omega, act);
+    launch_mg_matvec<kMgPost>(I, gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
     ++launches;
   } else
-    launch_mg_matvec<kMgPost>(gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
+    launch_mg_matvec<kMgPost>(I, gw, sl, s, tsw, dl, sv, bi, b, t, z, P.omega, act);
   if (fine) I.end(kcMgPost, q, mb + vb + vb / 12, mf);     // t in, z out (mb), b in, D^-1
   if (!fine) I.end(kcMgCoarse, q1, 0, 0);
   launches += 2;
@@ -1733,7 +1752,7 @@ int run_cg(DeviceSolver::Impl& I, int ndom, const Work& W, T* x, T* r, T* p, T* 
           q = I.begin(0);
           if (sizeof(T) == 4 && NEN == 8 && I.tensor_matvec)
             launch_sweep_tc(kTcApply, ti, nti, dd, I.svox(), fl, nullptr, nullptr, (const float*)p,
-                            (float*)w, 1.0f, 0.0f, pw, act, B<int>(I, bErr), s);
+                            (float*)w, 1.0f, 0.0f, pw, act, I.tc, s);
           else
             apply_k<T, NEN, false, true>(Wc, dd, I.svox(), fl, p, w, 1.0, pw, act, s);
           I.end(f32 ? kcMatvec32 : kcMatvec64, q, mb, mf);
@@ -1827,7 +1846,7 @@ int run_cg_mg(DeviceSolver::Impl& I, int ndom, int nactive, const Work& W, const
         int q = I.begin(0);
         if (NEN == 8 && I.tensor_matvec)
           launch_sweep_tc(kTcApply, Wc.ti, Wc.nti, dd, I.svox(), fl, nullptr, nullptr, p, w, 1.0f, 0.0f, nullptr,
-                          act, B<int>(I, bErr), s);
+                          act, I.tc, s);
         else
           apply_k<float, NEN, false, false>(Wc, dd, I.svox(), fl, p, w, 1.0, nullptr, act, s);
         I.end(kcMatvec32, q, mb, mf);
@@ -1970,16 +1989,16 @@ int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, co
     auto launch = [&]() {
       if (nen == 20) {
         if (cand == 0)
-          launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, M.doms0, M.svox0, M.flags0, *M.ke32, M.t0,
+          launch_hex20<float, false, false>(M.bricks0, M.nbricks0, M.layers0, M.doms0, M.svox0, M.flags0, I.k20_32, M.t0,
                                             M.z0, -1.0, nullptr, nullptr, s);
         else
           launch_ebe_tc(M.tcbricks0, M.ntcbricks0, M.doms0, M.svox0, M.flags0, W.ke20tc, M.t0, M.z0, -1.0, nullptr,
-                        nullptr, M.err, s);
+                        nullptr, I.tc, s);
       } else if (cand == 0) {
-        launch_mg_matvec<kMgPost>(gw, sl, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
+        launch_mg_matvec<kMgPost>(I, gw, sl, s, tsw, M.doms0, M.svox0, M.binv0, b, M.t0, M.z0, M.P->omega0, nullptr);
       } else {
         launch_sweep_tc(kTcPost, tsm, nsm, M.doms0, M.svox0, M.flags0, M.binv0, b, M.t0, M.z0, 1.0f, M.P->omega0,
-                        nullptr, nullptr, M.err, s);
+                        nullptr, nullptr, I.tc, s);
       }
     };
     if ((e = time_launches(s, launch, r.ms[cand], msg))) return e;
@@ -2227,39 +2246,41 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   I.pending.clear();
   I.h_active.clear();
   I.dom_mv_bytes.clear(); I.dom_mv_flops.clear(); I.dom_vec_bytes.clear();
-  // constant tables
+  // the solve's matrices
+  NodeBlocks<8> nb8;
+  NodeBlocks<NEN> nb;
   {
     double kh[576];
-    double wh[kWhNum];
-    float2 wh32[kWhNum];
     voxel_stiffness(8, nu, kh);
+    double wh[kWhNum];
     hadamard_entries(kh, wh);
-    for (int i = 0; i < kWhNum; ++i) wh32[i] = make_float2((float)wh[i], (float)wh[i]);
-    float kh32[576];
-    for (int i = 0; i < 576; ++i) kh32[i] = (float)kh[i];
-    DTC_CUDA(cudaMemcpyToSymbolAsync(c_khat64, kh, sizeof(kh), 0, cudaMemcpyHostToDevice, s));
-    DTC_CUDA(cudaMemcpyToSymbolAsync(c_kh32, kh32, sizeof(kh32), 0, cudaMemcpyHostToDevice, s));
-    DTC_CUDA(cudaMemcpyToSymbolAsync(c_wh64, wh, sizeof(wh), 0, cudaMemcpyHostToDevice, s));
-    DTC_CUDA(cudaMemcpyToSymbolAsync(c_wh32, wh32, sizeof(wh32), 0, cudaMemcpyHostToDevice, s));
-    if (int e = upload_tc_operand(kh, s, msg)) return e;
-    if (I.tensor_matvec || tune) {
-      if (int e = set_tc_spin_limit(opt.tc_wait_spins, s, msg)) return e;
-      if (int e = allow_sweep_tc(msg)) return e;
+    for (int i = 0; i < 576; ++i) {
+      I.kh64.v[i] = kh[i];
+      I.kh32.v[i] = (float)kh[i];
     }
-    if (NEN == 20) {
-      std::vector<double> k20(3600);
+    for (int i = 0; i < kWhNum; ++i) {
+      I.wh64.w[i] = wh[i];
+      I.wh32.w[i] = make_float2((float)wh[i], (float)wh[i]);
+    }
+    nb8 = node_blocks<8>(kh);
+    std::vector<double> k20(3600);
+    if constexpr (NEN == 20) {
       voxel_stiffness(20, nu, k20.data());
-      DTC_CUDA(cudaMemcpyToSymbolAsync(c_k20_64, k20.data(), sizeof(double) * 3600, 0, cudaMemcpyHostToDevice, s));
       I.k20_64 = class_blocks<double>(k20.data());
       I.k20_32 = class_blocks<float>(k20.data());
-      if (I.tensor_matvec || tune) {   // HEX20 FP32 applications on the tensor cores
-        std::vector<float> img(tc20_operand_bytes() / sizeof(float));
-        build_tc20_operand(k20.data(), img.data());
-        if (int e = ensure(I, bKe20tc, tc20_operand_bytes(), msg)) return e;
-        DTC_CUDA(cudaMemcpyAsync(I.bufs[bKe20tc], img.data(), tc20_operand_bytes(), cudaMemcpyHostToDevice, s));
-        if (int e = allow_ebe_tc(msg)) return e;
-      }
-      DTC_CUDA(cudaStreamSynchronize(s));   // the host vectors go out of scope
+      nb = node_blocks<20>(k20.data());
+    } else {
+      nb = nb8;
+    }
+    if (I.tensor_matvec || tune) {   // FP32 applications on the tensor cores
+      std::vector<float> img(NEN == 20 ? tc20_operand_bytes() / sizeof(float) : tc_operand_bytes() / sizeof(float));
+      if (NEN == 20) build_tc20_operand(k20.data(), img.data());
+      else build_tc_operand(kh, img.data());
+      const int slot = NEN == 20 ? bKe20tc : bKhTc;
+      if (int e = ensure(I, slot, sizeof(float) * img.size(), msg)) return e;
+      DTC_CUDA(cudaMemcpyAsync(I.bufs[slot], img.data(), sizeof(float) * img.size(), cudaMemcpyHostToDevice, s));
+      DTC_CUDA(cudaStreamSynchronize(s));   // the host vector goes out of scope
+      if (int e = NEN == 20 ? allow_ebe_tc(msg) : allow_sweep_tc(msg)) return e;
     }
     if (int e = allow_all_sweeps(msg)) return e;   // per device, cheap
     if (NEN == 20)
@@ -2339,6 +2360,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   if (energy && ncp > 1 && (e = ensure(I, bXkeep, vbytes64 * (ncp - 1), msg))) return e;
   if ((e = ensure(I, bErr, sizeof(int), msg))) return e;
   DTC_CUDA(cudaMemsetAsync(I.bufs[bErr], 0, sizeof(int), s));
+  I.tc = TcCtl{B<float>(I, bKhTc), tc_spin_limit(opt.tc_wait_spins), B<int>(I, bErr)};
 
   stats_.kc[kcHostPack].ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tpack).count();
   stats_.kc[kcHostPack].launches += 1;
@@ -2385,8 +2407,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   const Tile* ta = B<Tile>(I, bTilesA);
   const float* ke20tc = (NEN == 20 && (I.tensor_matvec || tune)) ? B<float>(I, bKe20tc) : nullptr;
   Work W{ti, ta, B<Tile>(I, bBricksI), B<Tile>(I, bBricksA), nti, nta, nbi, nba,
-               B<int64_t>(I, bNodesI), (int64_t)nodes_i.size(), &I.k20_64,
-               &I.k20_32, hb.layers, ke20tc, B<int>(I, bErr)};
+               B<int64_t>(I, bNodesI), (int64_t)nodes_i.size(), hb.layers, ke20tc, &I};
   W.bt = B<Tile>(I, bBricksTc);
   W.nbt = nbt;
   W.tw = B<Tile>(I, bTilesW);
@@ -2408,7 +2429,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   if (nta) {
     DTC_CUDA(cudaMemsetAsync(I.bufs[bBinv32], 0, sizeof(float) * node_total * 6, s));
     k_node_setup<NEN><<<(unsigned)nta, kThreads, 0, s>>>(ta, dd, I.svox(), fl, B<double>(I, bDinv64),
-                                                    B<float>(I, bDinv32), B<float>(I, bBinv32));
+                                                    B<float>(I, bDinv32), B<float>(I, bBinv32), nb);
     ++L;
   }
   if ((e = launch_check(msg))) return e;
@@ -2473,7 +2494,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
       if (mgp.all_n[l] > 0) {
         k_node_setup<8><<<(unsigned)mgp.all_n[l], kThreads, 0, s>>>(
             B<Tile>(I, bMgTiles) + mgp.all_off[l], B<DomDev>(I, bMgDoms) + (size_t)l * ndom, B<float>(I, bMgSvox),
-            B<uint8_t>(I, bMgFlags), B<double>(I, bMgDinv64), B<float>(I, bMgDinv32), B<float>(I, bMgBinv32));
+            B<uint8_t>(I, bMgFlags), B<double>(I, bMgDinv64), B<float>(I, bMgDinv32), B<float>(I, bMgBinv32), nb8);
         ++L;
       }
     if ((e = launch_check(msg))) return e;
@@ -2504,9 +2525,7 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
     mgd.ntcbricks0 = W.nbt;
     mgd.nodes0 = W.nodes;
     mgd.nnodes0 = W.nnodes;
-    mgd.ke32 = W.ke32;
     mgd.ke20tc = W.ke20tc;
-    mgd.err = W.err;
     if (tune) {
       if ((e = autotune_sweep(I, stats_, W, mgd, doms, svox, NEN, msg))) return e;
       if (!I.tensor_matvec) W.ke20tc = mgd.ke20tc = nullptr;   // HEX20: the column kernel won
@@ -2517,14 +2536,15 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
   }
 
   // the boundary modes (eps = 1e-6, the hard-coded boundary displacement of
-  // mod_write_deck.f90:61) and, per column pass, its 24 columns in c_uu
-  std::vector<double> modes((size_t)nm * 3 * nl), slices((size_t)ncp * 20 * 3 * kNLC, 0.0);
+  // mod_write_deck.f90:61) and, per column pass, its 24 columns
+  std::vector<double> modes((size_t)nm * 3 * nl);
+  std::vector<MacroModes> slices((size_t)ncp, MacroModes{});
   macro_modes_of_order(order, 1e-6, modes.data());
   for (int cp = 0; cp < ncp; ++cp)
     for (int lc = 0; lc < kNLC && cp * kNLC + lc < nl; ++lc)
       for (int c = 0; c < 3; ++c)
         for (int l = 0; l < nm; ++l)
-          slices[(size_t)cp * 20 * 3 * kNLC + l + nm * c + 3 * nm * lc] = modes[l + nm * c + (size_t)3 * nm * (cp * kNLC + lc)];
+          slices[cp].uu[l + nm * c + 3 * nm * lc] = modes[l + nm * c + (size_t)3 * nm * (cp * kNLC + lc)];
   bool want_fields = false;
   for (int d = 0; d < ndom; ++d) want_fields = want_fields || tasks[tidx[d]].out->displ || tasks[tidx[d]].out->force;
   std::vector<ColState> cs(ncol * ncp);
@@ -2543,11 +2563,9 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
         }
       }
     }
-    DTC_CUDA(cudaMemcpyToSymbolAsync(c_uu, slices.data() + (size_t)cp * 20 * 3 * kNLC, sizeof(double) * 20 * 3 * kNLC,
-                                     0, cudaMemcpyHostToDevice, s));
     if (nta) {
-      if (order == 2) k_boundary_values<20><<<(unsigned)nta, kThreads, 0, s>>>(ta, dd, fl, X);
-      else k_boundary_values<8><<<(unsigned)nta, kThreads, 0, s>>>(ta, dd, fl, X);
+      if (order == 2) k_boundary_values<20><<<(unsigned)nta, kThreads, 0, s>>>(ta, dd, fl, X, slices[cp]);
+      else k_boundary_values<8><<<(unsigned)nta, kThreads, 0, s>>>(ta, dd, fl, X, slices[cp]);
       ++L;
     }
     if ((e = launch_check(msg))) return e;
@@ -2850,7 +2868,8 @@ __global__ void k_adj_mix(const int64_t* __restrict__ blocks, const DomDev* __re
 // derivative of the energy products u_a^T K u_b (self-adjoint operator, so no adjoint solve).
 __global__ void k_energy_grad(const int64_t* __restrict__ blocks, const DomDev* __restrict__ doms,
                               const float* __restrict__ svox, const double* __restrict__ X,
-                              const double* __restrict__ V, float* __restrict__ grad) {
+                              const double* __restrict__ V, float* __restrict__ grad,
+                              const __grid_constant__ VoxelMatrix<double> kh) {
   const int64_t e = blocks[2 * blockIdx.x], start = blocks[2 * blockIdx.x + 1];
   const DomDev D = doms[e];
   const int64_t nvox = (int64_t)D.L[0] * D.L[1] * D.L[2];
@@ -2877,7 +2896,7 @@ __global__ void k_energy_grad(const int64_t* __restrict__ blocks, const DomDev* 
     for (int i = 0; i < 24; ++i) {
       double r = 0.0;
 #pragma unroll
-      for (int j = 0; j < 24; ++j) r = fma(c_khat64[i + 24 * j], u[j], r);
+      for (int j = 0; j < 24; ++j) r = fma(kh.v[i + 24 * j], u[j], r);
       sum = fma(w[i], r, sum);
     }
   }
@@ -2999,7 +3018,7 @@ int DeviceSolver::energy_grad(const double* dloss_dc, float* const* grad_e, int6
                                                           B<double>(I, bAdjV));
     if (!vb.empty())
       k_energy_grad<<<(unsigned)(vb.size() / 2), 128, 0, s>>>(blocks + nb.size(), B<DomDev>(I, bAdjDoms), sv, X,
-                                                              B<double>(I, bAdjV), B<float>(I, bAdjGrad));
+                                                              B<double>(I, bAdjV), B<float>(I, bAdjGrad), I.kh64);
     if ((e = launch_check(msg))) return e;
     if (grad_on_device) {
       for (int d = 0; d < nd; ++d) {

@@ -42,6 +42,14 @@ __device__ __forceinline__ void block_jacobi(const float* __restrict__ binv, int
   z[2] = omega * (b4 * r[0] + b5 * r[1] + b2 * r[2]);
 }
 
+// What the tensor-core kernels need beside the vectors: the HEX08 operand (device memory), the polls of a
+// completion wait before it gives up, and the flag that records a wait that did.
+struct TcCtl {
+  const float* khat;
+  long long spins;
+  int* err;
+};
+
 // Epilogues of the tensor-core HEX08 sweep (matvec_tc.cu, launch_sweep_tc)
 enum { kTcApply = 0, kTcRes = 1, kTcPost = 2 };
 

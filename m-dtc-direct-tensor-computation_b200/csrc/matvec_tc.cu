@@ -97,16 +97,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
 
 }  // namespace tc
 
-// Polls of the per-round completion wait before a kernel gives up (the drain wait before the
-// tensor memory is freed always keeps the full bound).  dtc_options.tc_wait_spins sets it.
-__device__ long long g_tc_spin_limit = tc::kSpinLimit;
-
-int set_tc_spin_limit(long long spins, cudaStream_t s, std::string& msg) {
-  const long long v = spins > 0 ? spins : spins == 0 ? tc::kSpinLimit : 0;
-  DTC_CUDA(cudaMemcpyToSymbolAsync(g_tc_spin_limit, &v, sizeof(v), 0, cudaMemcpyHostToDevice, s));
-  DTC_CUDA(cudaStreamSynchronize(s));   // v lives on this stack frame
-  return DTC_OK;
-}
+// Polls of the per-round completion wait before a kernel gives up, from dtc_options.tc_wait_spins (the drain wait
+// before the tensor memory is freed always keeps the full bound).
+long long tc_spin_limit(long long spins) { return spins > 0 ? spins : spins == 0 ? tc::kSpinLimit : 0; }
 
 // -------------------------------------------------------------------------------------
 // HEX08 sweeps of the FP32 inner solve on the tensor cores.
@@ -128,7 +121,7 @@ int set_tc_spin_limit(long long spins, cudaStream_t s, std::string& msg) {
 //   kTcPost : y = u + omega D^-1 (b - K u)                   (post-smoothing)
 // Precision: the split recovers FP32-level products (the tf32 rounding of the lo parts costs
 // at most 2^-21 relative); accumulation is FP32 in tensor memory, then FP64 for the scale.
-// Waits: every completion wait is bounded by g_tc_spin_limit polls; on time-out the CTA
+// Waits: every completion wait is bounded by ctl.spins polls; on time-out the CTA
 // records the error, waits (full bound) for the MMAs it committed, frees its tensor memory
 // and returns.
 namespace tc {
@@ -178,16 +171,14 @@ __device__ __forceinline__ int corner_dy(int lm) { return (lm == 2 || lm == 3 ||
 __device__ __forceinline__ int corner_dz(int lm) { return lm >= 4 ? 1 : 0; }
 }  // namespace tc
 
-// Khat split into tf32 hi / lo, laid out as 6 canonical B chunks (hi k0..2, lo k0..2).
-__constant__ float c_bsplit[6 * tc::kN * tc::kKc];
+// ctl.khat: Khat split into tf32 hi / lo, laid out as 6 canonical B chunks (hi k0..2, lo k0..2).
 
 template <int MODE>
 __global__ void __launch_bounds__(128, 4)
     k_sweep_tc(const Tile* __restrict__ tiles, const DomDev* __restrict__ doms, const float* __restrict__ svox,
                const uint8_t* __restrict__ flags, const float* __restrict__ binv, const float* __restrict__ b,
                const float* __restrict__ u, float* __restrict__ y, float scale, float omega,
-               double* __restrict__ dots, const int* __restrict__ dom_active,
-               int* __restrict__ err) {
+               double* __restrict__ dots, const int* __restrict__ dom_active, const TcCtl ctl) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char dsm[];
   unsigned char* sB = dsm;                                        // 6 KB, canonical K-major chunks
@@ -217,7 +208,7 @@ __global__ void __launch_bounds__(128, 4)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
-  for (int i = tid; i < 6 * kN * kKc; i += 128) reinterpret_cast<float*>(sB)[i] = c_bsplit[i];
+  for (int i = tid; i < 6 * kN * kKc; i += 128) reinterpret_cast<float*>(sB)[i] = __ldg(ctl.khat + i);
   for (int i = tid; i < 128 * 3 * 8; i += 128) acc[i] = 0.0f;
 
   // kept voxels adjacent to the owned nodes, in x-fastest order
@@ -268,7 +259,7 @@ __global__ void __launch_bounds__(128, 4)
   const uint32_t sB_addr = smem_u32(sB);
   const int lcl = tid & 7, lc = g * kLcGroup + lcl;
   const int rounds = (nv + kSweepVox - 1) / kSweepVox;
-  const long long lim = g_tc_spin_limit;
+  const long long lim = ctl.spins;
   const int64_t nx = D.n[0], nxy = (int64_t)D.n[0] * D.n[1];
   const int hi_x = D.n[0] - 2, hi_y = D.n[1] - 2, hi_z = D.n[2] - 2;
 
@@ -357,7 +348,7 @@ __global__ void __launch_bounds__(128, 4)
     }
   }
   if (fail) {
-    if (tid == 0) atomicExch(err, 1);
+    if (tid == 0) atomicExch(ctl.err, 1);
     // bounded with the full limit: wait for the last committed MMAs before freeing their memory
     if (committed > 0) mbar_wait(smem_u32(&mbar), (uint32_t)((committed - 1) & 1));
   }
@@ -423,24 +414,24 @@ int allow_sweep_tc(std::string& msg) {
 
 void launch_sweep_tc(int mode, const Tile* tiles, int64_t ntiles, const DomDev* doms, const float* svox,
                      const uint8_t* flags, const float* binv, const float* b, const float* u, float* y, float scale,
-                     float omega, double* dots, const int* dom_active, int* err, cudaStream_t s) {
+                     float omega, double* dots, const int* dom_active, const TcCtl& ctl, cudaStream_t s) {
   if (ntiles <= 0) return;
   const unsigned grid = (unsigned)(3 * ntiles);
   if (mode == kTcApply)
     k_sweep_tc<kTcApply><<<grid, 128, tc::kSweepSmem, s>>>(tiles, doms, svox, flags, binv, b, u, y, scale, omega,
-                                                            dots, dom_active, err);
+                                                            dots, dom_active, ctl);
   else if (mode == kTcRes)
     k_sweep_tc<kTcRes><<<grid, 128, tc::kSweepSmem, s>>>(tiles, doms, svox, flags, binv, b, u, y, scale, omega, dots,
-                                                          dom_active, err);
+                                                          dom_active, ctl);
   else
     k_sweep_tc<kTcPost><<<grid, 128, tc::kSweepSmem, s>>>(tiles, doms, svox, flags, binv, b, u, y, scale, omega,
-                                                           dots, dom_active, err);
+                                                           dots, dom_active, ctl);
 }
 
-// Host: build the split Khat in the canonical B layout and upload it.
-int upload_tc_operand(const double* khat, cudaStream_t s, std::string& msg) {
+// Host: the split Khat in the canonical B layout.
+size_t tc_operand_bytes() { return sizeof(float) * 6 * tc::kN * tc::kKc; }
+void build_tc_operand(const double* khat, float* img) {
   using namespace tc;
-  float img[6 * kN * kKc];
   for (int i = 0; i < 6 * kN * kKc; ++i) img[i] = 0.0f;
   for (int n = 0; n < 24; ++n)
     for (int k = 0; k < kK; ++k) {
@@ -461,8 +452,6 @@ int upload_tc_operand(const double* khat, cudaStream_t s, std::string& msg) {
       img[(kc * kBChunkBytes + canon_offset(n, kk)) / 4] = hi;
       img[((3 + kc) * kBChunkBytes + canon_offset(n, kk)) / 4] = lo;
     }
-  DTC_CUDA(cudaMemcpyToSymbolAsync(c_bsplit, img, sizeof(img), 0, cudaMemcpyHostToDevice, s));
-  return DTC_OK;
 }
 
 // -------------------------------------------------------------------------------------
@@ -516,7 +505,7 @@ __global__ void __launch_bounds__(128, 2)
     k_ebe_tc(const Tile* __restrict__ bricks, const DomDev* __restrict__ doms, const float* __restrict__ svox,
              const uint8_t* __restrict__ flags, const float* __restrict__ bsplit, const float* __restrict__ u,
              float* __restrict__ y, double scale, double* __restrict__ acc_pw, const int* __restrict__ dom_active,
-             int* __restrict__ err) {
+             const TcCtl ctl) {
   using namespace tc20;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -615,7 +604,7 @@ __global__ void __launch_bounds__(128, 2)
   const uint32_t sB_addr = tc::smem_u32(sB);
   const int l = tid & (kLcg - 1);
   const int rounds = (nv + kVoxPerRound - 1) / kVoxPerRound;
-  const long long lim = g_tc_spin_limit;
+  const long long lim = ctl.spins;
   // staged-grid offset of ring node a relative to the voxel's node 0
   auto ring_off = [](int a) { return kRing[a][0] + kIx * (kRing[a][1] + kIy * kRing[a][2]); };
 
@@ -697,7 +686,7 @@ __global__ void __launch_bounds__(128, 2)
     }
   }
   if (fail) {
-    if (tid == 0) atomicExch(err, 1);
+    if (tid == 0) atomicExch(ctl.err, 1);
     // bounded with the full limit: wait for the last committed MMAs before freeing their memory
     if (committed > 0) tc::mbar_wait(tc::smem_u32(&mbar), (uint32_t)((committed - 1) & 1));
   }
@@ -768,15 +757,15 @@ int allow_ebe_tc(std::string& msg) {
 
 void launch_ebe_tc(const Tile* bricks, int64_t nb, const DomDev* doms, const float* svox, const uint8_t* flags,
                    const float* bsplit, const float* u, float* y, double scale, double* acc_pw, const int* dom_active,
-                   int* err, cudaStream_t s) {
+                   const TcCtl& ctl, cudaStream_t s) {
   if (nb <= 0) return;
   const unsigned grid = (unsigned)((kNLC / tc20::kLcg) * nb);
   if (acc_pw)
     k_ebe_tc<true><<<grid, 128, tc20::kSmem, s>>>(bricks, doms, svox, flags, bsplit, u, y, scale, acc_pw, dom_active,
-                                                  err);
+                                                  ctl);
   else
     k_ebe_tc<false><<<grid, 128, tc20::kSmem, s>>>(bricks, doms, svox, flags, bsplit, u, y, scale, nullptr,
-                                                   dom_active, err);
+                                                   dom_active, ctl);
 }
 
 }  // namespace dtc

@@ -64,7 +64,7 @@ struct MRes {
   int32_t last_vox;    // voxel of the last element
 };
 
-__constant__ signed char c_mloc[20][3];   // local node offsets: HEX08 corners or HEX20 ring
+struct NodeOffsets { signed char a[20][3]; };   // of an element's nodes: HEX08 corners or HEX20 ring
 
 __device__ __forceinline__ int64_t gray_at(const unsigned char* phi, const MDom& D, int64_t v) {
   const unsigned char* p = phi + D.phi_off;
@@ -230,7 +230,8 @@ __global__ void k_compress(const int64_t* __restrict__ blk, const MDom* __restri
 __global__ void k_kept_keys(const int64_t* __restrict__ blk, const MDom* __restrict__ doms,
                             const uint8_t* __restrict__ bone, const int32_t* __restrict__ elem_of,
                             const int32_t* __restrict__ par, const uint8_t* __restrict__ keepc,
-                            uint8_t* __restrict__ kept, int32_t* __restrict__ key, MRes* __restrict__ res) {
+                            uint8_t* __restrict__ kept, int32_t* __restrict__ key, MRes* __restrict__ res,
+                            const __grid_constant__ NodeOffsets loc) {
   const int64_t d = blk[2 * blockIdx.x], v = blk[2 * blockIdx.x + 1] + threadIdx.x;
   const MDom D = doms[d];
   const int64_t nv = (int64_t)D.L[0] * D.L[1] * D.L[2];
@@ -241,8 +242,8 @@ __global__ void k_kept_keys(const int64_t* __restrict__ blk, const MDom* __restr
     const int32_t e = elem_of[D.vox_off + v];
     const int x = (int)(v % D.L[0]), y = (int)((v / D.L[0]) % D.L[1]), z = (int)(v / ((int64_t)D.L[0] * D.L[1]));
     for (int a = 0; a < D.nen; ++a) {
-      const int64_t g = (D.m * x + c_mloc[a][0]) + (int64_t)D.g[0] * ((D.m * y + c_mloc[a][1]) +
-                                                                      (int64_t)D.g[1] * (D.m * z + c_mloc[a][2]));
+      const int64_t g = (D.m * x + loc.a[a][0]) + (int64_t)D.g[0] * ((D.m * y + loc.a[a][1]) +
+                                                                      (int64_t)D.g[1] * (D.m * z + loc.a[a][2]));
       atomicMin(&key[D.node_off + g], e * D.nen + a);
     }
   } else if (v < nv) {
@@ -286,7 +287,8 @@ __global__ void k_nodes(const int64_t* __restrict__ blk, const MDom* __restrict_
 __global__ void k_slot_flags(const int64_t* __restrict__ blk, const MDom* __restrict__ doms,
                              const MRes* __restrict__ res, const int32_t* __restrict__ key,
                              const int32_t* __restrict__ evox, const uint8_t* __restrict__ node_keep,
-                             int32_t* __restrict__ flag, int64_t* __restrict__ slot_grid) {
+                             int32_t* __restrict__ flag, int64_t* __restrict__ slot_grid,
+                             const __grid_constant__ NodeOffsets loc) {
   const int64_t d = blk[2 * blockIdx.x], s = blk[2 * blockIdx.x + 1] + threadIdx.x;
   const MDom D = doms[d];
   const MRes R = res[d];
@@ -295,8 +297,8 @@ __global__ void k_slot_flags(const int64_t* __restrict__ blk, const MDom* __rest
   const int32_t e = (int32_t)(s / D.nen), a = (int32_t)(s % D.nen);
   const int32_t v = evox[D.elem_off + e];
   const int x = (int)(v % D.L[0]), y = (int)((v / D.L[0]) % D.L[1]), z = (int)(v / ((int64_t)D.L[0] * D.L[1]));
-  const int64_t g = (D.m * x + c_mloc[a][0]) + (int64_t)D.g[0] * ((D.m * y + c_mloc[a][1]) +
-                                                                  (int64_t)D.g[1] * (D.m * z + c_mloc[a][2]));
+  const int64_t g = (D.m * x + loc.a[a][0]) + (int64_t)D.g[0] * ((D.m * y + loc.a[a][1]) +
+                                                                  (int64_t)D.g[1] * (D.m * z + loc.a[a][2]));
   slot_grid[D.slot_off + s] = g;
   const bool first = key[D.node_off + g] == (int32_t)s;
   flag[D.slot_off + s] = first && (node_keep[D.node_off + g] || (int32_t)s == R.last_key);
@@ -400,10 +402,8 @@ int mesh_batch_device(const dtc_domain_in* in, int64_t n, MeshPlan* plans, bool 
       msg = "device mesher: domain too large for 32-bit first-appearance keys";
       return DTC_ERR_INVALID_ARGUMENT;
     }
-  signed char loc[20][3];
-  std::memset(loc, 0, sizeof(loc));
-  std::memcpy(loc, nen == 8 ? &kCorner[0][0] : &kRing[0][0], (size_t)nen * 3);
-  DTC_CUDA(cudaMemcpyToSymbolAsync(c_mloc, loc, sizeof(loc), 0, cudaMemcpyHostToDevice, s));
+  NodeOffsets loc = {};
+  std::memcpy(loc.a, nen == 8 ? &kCorner[0][0] : &kRing[0][0], (size_t)nen * 3);
   const int m = nen == 8 ? 1 : 2;
   std::vector<MDom> doms((size_t)n);
   int64_t vox = 0, nodes = 0, phib = 0;
@@ -480,7 +480,7 @@ int mesh_batch_device(const dtc_domain_in* in, int64_t n, MeshPlan* plans, bool 
   k_keep<<<nvb, kMB, 0, s>>>(dvblk, ddoms, dres, bone, elem_of, par, keepc);
   k_compress<<<nvb, kMB, 0, s>>>(dvblk, ddoms, bone, par);
   if ((e = cudaGetLastError())) return fail(e, "components");
-  k_kept_keys<<<nvb, kMB, 0, s>>>(dvblk, ddoms, bone, elem_of, par, keepc, kept, key, dres);
+  k_kept_keys<<<nvb, kMB, 0, s>>>(dvblk, ddoms, bone, elem_of, par, keepc, kept, key, dres, loc);
   k_nodes<<<nnb, kMB, 0, s>>>(dnblk, ddoms, key, evox, par, keepc, node_keep, dres);
   if ((e = cudaGetLastError())) return fail(e, "nodes");
   std::vector<MRes> hres((size_t)n);
@@ -511,7 +511,7 @@ int mesh_batch_device(const dtc_domain_in* in, int64_t n, MeshPlan* plans, bool 
     const int32_t lk = R.last_key;
     const int32_t a = lk % nen;
     const int64_t vx = vlast % D.L[0], vy = (vlast / D.L[0]) % D.L[1], vz = vlast / ((int64_t)D.L[0] * D.L[1]);
-    const int64_t g = (m * vx + loc[a][0]) + (int64_t)D.g[0] * ((m * vy + loc[a][1]) + (int64_t)D.g[1] * (m * vz + loc[a][2]));
+    const int64_t g = (m * vx + loc.a[a][0]) + (int64_t)D.g[0] * ((m * vy + loc.a[a][1]) + (int64_t)D.g[1] * (m * vz + loc.a[a][2]));
     const int64_t ix = g % D.g[0], iy = (g / D.g[0]) % D.g[1], iz = g / ((int64_t)D.g[0] * D.g[1]);
     const bool lonb = ix == 0 || ix == D.g[0] - 1 || iy == 0 || iy == D.g[1] - 1 || iz == 0 || iz == D.g[2] - 1;
     if (!last_kept) {
@@ -566,7 +566,7 @@ int mesh_batch_device(const dtc_domain_in* in, int64_t n, MeshPlan* plans, bool 
       return fail(e, "numbering set-up");
     if (neb) k_elem_flags<<<(unsigned)neb, kMB, 0, s>>>(deblk, ddoms, dres, evox, kept, eflag);
     if (nsb) {
-      k_slot_flags<<<(unsigned)nsb, kMB, 0, s>>>(dsblk, ddoms, dres, key, evox, node_keep, sflag, sgrid);
+      k_slot_flags<<<(unsigned)nsb, kMB, 0, s>>>(dsblk, ddoms, dres, key, evox, node_keep, sflag, sgrid, loc);
       k_block_sums<<<(unsigned)nsb, kMB, 0, s>>>(dsblk, (int64_t)nsb, meta, meta + n, sflag, sbs);
       k_scan_blocks<<<(unsigned)n, 32, 0, s>>>(meta + 4 * n, meta + 5 * n, sbs);
       k_scan_items<<<(unsigned)nsb, kMB, 0, s>>>(dsblk, meta, meta + n, sflag, sbs, srank);

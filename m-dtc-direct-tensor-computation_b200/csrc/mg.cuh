@@ -291,7 +291,8 @@ constexpr int kTailSmem = 4 * kTailFloats + kTailItems / kTailLc;
 
 // sum over the 8 voxels around a node of s_v Khat (u - u(node)); u: the node's load case in the staged
 // vector, sv: its voxel on the low sides (stride 8)
-__device__ __forceinline__ void tail_apply(const float* u, const float* sv, float (&r)[3]) {
+__device__ __forceinline__ void tail_apply(const VoxelMatrix<float>& kh, const float* u, const float* sv,
+                                           float (&r)[3]) {
   constexpr int X = 3 * kTailLc, Y = kTailN * X, Z = kTailN * Y;
   float d[27][3];
 #pragma unroll
@@ -318,7 +319,7 @@ __device__ __forceinline__ void tail_apply(const float* u, const float* sv, floa
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) k[i] = fmaf(c_kh32[3 * a + i + 24 * (3 * e + j)], d[n][j], k[i]);
+        for (int j = 0; j < 3; ++j) k[i] = fmaf(kh.v[3 * a + i + 24 * (3 * e + j)], d[n][j], k[i]);
     }
     const float s = sv[vx + 8 * vy + 64 * vz];
 #pragma unroll
@@ -328,8 +329,8 @@ __device__ __forceinline__ void tail_apply(const float* u, const float* sv, floa
 
 __global__ void __launch_bounds__(kTailThreads, 1)
     k_mg_tail(const int* __restrict__ list, const DomDev* __restrict__ doms_f, const DomDev* __restrict__ doms_c,
-              const float* __restrict__ svox, const uint8_t* __restrict__ flags, const float* __restrict__ binv,
-              const float* __restrict__ minv, const float* __restrict__ b, float* __restrict__ z, float omega,
+              const float* __restrict__ svox, const __grid_constant__ VoxelMatrix<float> kh,
+              const uint8_t* __restrict__ flags, const float* __restrict__ binv, const float* __restrict__ minv, const float* __restrict__ b, float* __restrict__ z, float omega,
               int steps, const int* __restrict__ dom_active) {
   extern __shared__ __align__(16) unsigned char tail_smem[];
   constexpr int kNodes = kTailItems / kTailLc, NT = kTailThreads;
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(kTailThreads, 1)
   for (int step = 0; step < steps; ++step) {
     nodes([&](int n, int i, int x, int y, int zz, int k) {
       float r[3], v[3];
-      tail_apply(src + k, sv + (x - 1) + 8 * (y - 1) + 64 * (zz - 1), r);
+      tail_apply(kh, src + k, sv + (x - 1) + 8 * (y - 1) + 64 * (zz - 1), r);
       for (int c = 0; c < 3; ++c) r[c] = sb[3 * i + c] - r[c];
       if (step == turn) {
         for (int c = 0; c < 3; ++c) dst[k + c * kTailLc] = r[c];

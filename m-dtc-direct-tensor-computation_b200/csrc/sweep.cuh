@@ -27,8 +27,8 @@ static_assert(kVoxRows * 4 <= kSweepThreads, "one thread per voxel row and 8 byt
 // the normal strains), shear, the corner mode, the same two for the classes that are odd in one axis,
 // and for the class that is odd in all three.
 enum { kWhAxD, kWhAxO, kWhSh, kWhCo, kWhOneD, kWhOneO, kWhAllD, kWhAllO, kWhNum };
-__constant__ float2 c_wh32[kWhNum];
-__constant__ double c_wh64[kWhNum];
+template <typename T> struct Hadamard { T w[kWhNum]; };
+template <> struct Hadamard<float> { float2 w[kWhNum]; };   // twice: an operand of packed arithmetic
 
 // The entries from the voxel matrix (column-major 24 x 24): g_b^T K g_a / 64 with g the +-1 corner patterns.
 inline void hadamard_entries(const double* khat, double (&w)[kWhNum]) {
@@ -65,7 +65,7 @@ template <> struct Lane<float> {
   static __device__ __forceinline__ V sub(V a, V b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
   static __device__ __forceinline__ V mul(V a, V b) { return __fmul2_rn(a, b); }
   static __device__ __forceinline__ V fma(V a, V b, V c) { return __ffma2_rn(a, b, c); }
-  static __device__ __forceinline__ V coef(int i, float s) { return __fmul2_rn(c_wh32[i], make_float2(s, s)); }
+  static __device__ __forceinline__ V coef(V w, float s) { return __fmul2_rn(w, make_float2(s, s)); }
   static __device__ __forceinline__ V load(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
   static __device__ __forceinline__ void store(float* p, V v) { *reinterpret_cast<float2*>(p) = v; }
   // v * scale with the FP64 scale as two floats: within one rounding of the product
@@ -87,7 +87,7 @@ template <> struct Lane<double> {
   static __device__ __forceinline__ V sub(V a, V b) { return a - b; }
   static __device__ __forceinline__ V mul(V a, V b) { return a * b; }
   static __device__ __forceinline__ V fma(V a, V b, V c) { return ::fma(a, b, c); }
-  static __device__ __forceinline__ V coef(int i, float s) { return c_wh64[i] * (double)s; }
+  static __device__ __forceinline__ V coef(V w, float s) { return w * (double)s; }
   static __device__ __forceinline__ V load(const double* p) { return __ldg(p); }
   static __device__ __forceinline__ void store(double* p, V v) { *p = v; }
   struct Scale {
@@ -132,7 +132,8 @@ template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.
 // class, so that few of the 21 sums and differences live at a time.
 template <typename T>
 __device__ __forceinline__ void wh_voxel(const typename Lane<T>::V (&p)[4][3], const typename Lane<T>::V (&q)[4][3],
-                                         float s, typename Lane<T>::V (&f)[4][3], typename Lane<T>::V (&g)[4][3]) {
+                                         const Hadamard<T>& W, float s, typename Lane<T>::V (&f)[4][3],
+                                         typename Lane<T>::V (&g)[4][3]) {
   using L = Lane<T>;
   using V = typename L::V;
   auto sum = [&](int b, int c) { return L::add(q[b][c], p[b][c]); };
@@ -142,10 +143,10 @@ __device__ __forceinline__ void wh_voxel(const typename Lane<T>::V (&p)[4][3], c
   auto even2 = [&](int b, int c, V v) { f[b][c] = L::add(f[b][c], v); g[b][c] = L::add(g[b][c], v); };
   auto odd1 = [&](int b, int c, V v) { f[b][c] = L::sub(f[b][c], v); g[b][c] = v; };
   auto odd2 = [&](int b, int c, V v) { f[b][c] = L::sub(f[b][c], v); g[b][c] = L::add(g[b][c], v); };
-  const V one_d = L::coef(kWhOneD, s), one_o = L::coef(kWhOneO, s), sh = L::coef(kWhSh, s);
+  const V one_d = L::coef(W.w[kWhOneD], s), one_o = L::coef(W.w[kWhOneO], s), sh = L::coef(W.w[kWhSh], s);
   {   // normal strains
     const V a = dif(0, 0), b = sum(1, 1), c = sum(2, 2);
-    const V d = L::coef(kWhAxD, s), t = L::mul(L::coef(kWhAxO, s), L::add(L::add(a, b), c));
+    const V d = L::coef(W.w[kWhAxD], s), t = L::mul(L::coef(W.w[kWhAxO], s), L::add(L::add(a, b), c));
     odd1(0, 0, L::fma(d, a, t));
     even1(1, 1, L::fma(d, b, t));
     even1(2, 2, L::fma(d, c, t));
@@ -176,13 +177,13 @@ __device__ __forceinline__ void wh_voxel(const typename Lane<T>::V (&p)[4][3], c
     even1(2, 1, m);
     even1(1, 2, m);
     const V a = sum(3, 0), b = dif(2, 1), c = dif(1, 2);
-    const V d = L::coef(kWhAllD, s), t = L::mul(L::coef(kWhAllO, s), L::add(L::add(a, b), c));
+    const V d = L::coef(W.w[kWhAllD], s), t = L::mul(L::coef(W.w[kWhAllO], s), L::add(L::add(a, b), c));
     even1(3, 0, L::fma(d, a, t));
     odd2(2, 1, L::fma(d, b, t));
     odd2(1, 2, L::fma(d, c, t));
   }
   {   // corner modes
-    const V e = L::coef(kWhCo, s);
+    const V e = L::coef(W.w[kWhCo], s);
 #pragma unroll
     for (int c = 0; c < 3; ++c) odd2(3, c, L::mul(e, dif(3, c)));
   }
@@ -228,6 +229,7 @@ template <typename T, bool ALL, int MODE>
 __global__ void __launch_bounds__(kSweepThreads, 2) k_sweep(const Tile* __restrict__ tiles, int len,
                                                             const DomDev* __restrict__ doms,
                                                             const float* __restrict__ svox,
+                                                            const __grid_constant__ Hadamard<T> W,
                                                             const T* __restrict__ u, T* __restrict__ y,
                                                             double scale, const float* __restrict__ binv,
                                                             const T* __restrict__ b, float omega,
@@ -343,7 +345,7 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_sweep(const Tile* __restri
     V q[4][3], g[4][3];                         // q holds nothing where no voxel needs it
     if ((kept >> i) & 3) wh_plane<T>(ring + next * kPlaneElems + corner, q);   // plane x + 1
     if ((kept >> i) & 1) {
-      wh_voxel<T>(p, q, fac[row * kStep + i], f, g);
+      wh_voxel<T>(p, q, W, fac[row * kStep + i], f, g);
     } else {
 #pragma unroll
       for (int a = 0; a < 4; ++a)

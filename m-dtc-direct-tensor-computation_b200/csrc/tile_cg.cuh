@@ -23,7 +23,7 @@ constexpr double kTightRtol = 1e-10;
 // corners' values from u, kb being the index of the row's value at plane x for its load case, and adds to node x
 // (corner offset 0 in x) and node x+1 (offset 1).  FIRST: only node x+1 belongs to the tile.
 template <bool FIRST>
-__device__ __forceinline__ void voxel_rd(const double* __restrict__ u, int64_t kb, int sy, int sz, int b, int c,
+__device__ __forceinline__ void voxel_rd(const VoxelMatrix<double>& kh, const double* __restrict__ u, int64_t kb, int sy, int sz, int b, int c,
                                          float s, double (&cur)[3], double (&nxt)[3]) {
   const int l0 = corner_local(0, 1 - b, 1 - c), l1 = corner_local(1, 1 - b, 1 - c);
   double t0 = 0, t1 = 0, t2 = 0, q0 = 0, q1 = 0, q2 = 0;
@@ -40,13 +40,13 @@ __device__ __forceinline__ void voxel_rd(const double* __restrict__ u, int64_t k
           const double v = __ldg(u + k + cj * kNLC);
           const int col = 24 * (3 * lm + cj);
           if (!FIRST) {
-            t0 = fma(c_khat64[col + 3 * l0 + 0], v, t0);
-            t1 = fma(c_khat64[col + 3 * l0 + 1], v, t1);
-            t2 = fma(c_khat64[col + 3 * l0 + 2], v, t2);
+            t0 = fma(kh.v[col + 3 * l0 + 0], v, t0);
+            t1 = fma(kh.v[col + 3 * l0 + 1], v, t1);
+            t2 = fma(kh.v[col + 3 * l0 + 2], v, t2);
           }
-          q0 = fma(c_khat64[col + 3 * l1 + 0], v, q0);
-          q1 = fma(c_khat64[col + 3 * l1 + 1], v, q1);
-          q2 = fma(c_khat64[col + 3 * l1 + 2], v, q2);
+          q0 = fma(kh.v[col + 3 * l1 + 0], v, q0);
+          q1 = fma(kh.v[col + 3 * l1 + 1], v, q1);
+          q2 = fma(kh.v[col + 3 * l1 + 2], v, q2);
         }
       }
   const double ts = (double)s;
@@ -67,6 +67,7 @@ template <bool DOT>
 __global__ void __launch_bounds__(kThreads, 4) k_tile_matvec(const Tile* __restrict__ tiles,
                                                              const DomDev* __restrict__ doms,
                                                              const float* __restrict__ svox,
+                                                             const __grid_constant__ VoxelMatrix<double> kh,
                                                              const double* __restrict__ u, double* __restrict__ y,
                                                              double scale, double* __restrict__ acc,
                                                              const int* __restrict__ dom_active, int bnd_only) {
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_tile_matvec(const Tile* __restr
     for (int b = 0; b < 2; ++b)
 #pragma unroll
       for (int c = 0; c < 2; ++c)
-        if (sv[b][c] != 0.f) voxel_rd<true>(u, kx, sy, sz, b, c, sv[b][c], cur, nxt);
+        if (sv[b][c] != 0.f) voxel_rd<true>(kh, u, kx, sy, sz, b, c, sv[b][c], cur, nxt);
 #pragma unroll 1
     for (int x = x0; x <= xe; ++x) {
       kx += 3 * kNLC;   // plane x
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_tile_matvec(const Tile* __restr
       for (int b = 0; b < 2; ++b)
 #pragma unroll
         for (int c = 0; c < 2; ++c)
-          if (sv[b][c] != 0.f) voxel_rd<false>(u, kx, sy, sz, b, c, sv[b][c], cur, nxt);
+          if (sv[b][c] != 0.f) voxel_rd<false>(kh, u, kx, sy, sz, b, c, sv[b][c], cur, nxt);
       if (anyp | anyc) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
