@@ -81,8 +81,8 @@ typedef struct dtc_options {
                               1 = tcgen05 tensor cores (3xTF32 split, FP32-level accuracy),
                               2 = autotuned: multigrid solves time both kernels of the fine-level
                               operator on the batch's own tiles and keep the faster; cached per
-                              device and size class (dtc_get_kernel_stats lists the timings as
-                              autotune_* classes) */
+                              device, size class and size of the launch (dtc_get_kernel_stats
+                              lists the timings as autotune_* classes) */
   int32_t inner_precond;   /* preconditioner of the FP32 inner solve: 0 = Jacobi (as PETSc's
                               PCJACOBI), 1 = node-block Jacobi (3x3 diagonal blocks),
                               2 = multigrid V-cycle on halved voxel grids (HEX20 domains are

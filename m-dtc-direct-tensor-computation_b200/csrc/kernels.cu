@@ -1898,12 +1898,14 @@ int run_cg_mg(DeviceSolver::Impl& I, int ndom, int nactive, const Work& W, const
 // Autotuner of the fine-level operator (mixed_matvec = 2): the SIMT kernel and the tcgen05 kernel run on the
 // batch's own tiles, one warm-up and three timed launches each (CUDA events on the solver stream); the faster
 // one serves the whole solve.  Choices are cached per device and size class -- the median domain edge (16, 24,
-// 32, 48, 64 voxels ...) and the kept-voxel fraction (below 0.15, 0.30, above) -- so later batches of the same
-// class skip the timing.
+// 32, 48, 64 voxels ...), the kept-voxel fraction (below 0.15, 0.30, above) and the launch -- the SIMT kernel's tile
+// length (HEX20: layers, to a power of two) and whether its CTAs take less than one wave of the card, up to four, or
+// more: what wins on one small domain says little about hundreds -- so later batches of the same class skip the timing.
 struct TuneKey {
-  int device, nen, lclass, fclass;
+  int device, nen, lclass, fclass, length, waves;
   bool operator<(const TuneKey& o) const {
-    return std::tie(device, nen, lclass, fclass) < std::tie(o.device, o.nen, o.lclass, o.fclass);
+    return std::tie(device, nen, lclass, fclass, length, waves) <
+           std::tie(o.device, o.nen, o.lclass, o.fclass, o.length, o.waves);
   }
 };
 struct TuneResult {
@@ -1943,7 +1945,7 @@ int time_launches(cudaStream_t s, F&& launch, float& ms, std::string& msg) {
   return launch_check(msg);
 }
 
-TuneKey tune_key(int device, int nen, const std::vector<DomDev>& doms, const std::vector<float>& svox) {
+TuneKey tune_key(int device, int nen, const Work& W, const std::vector<DomDev>& doms, const std::vector<float>& svox) {
   std::vector<int> Ls;
   for (const DomDev& D : doms) Ls.push_back(std::max(D.L[0], std::max(D.L[1], D.L[2])));
   std::nth_element(Ls.begin(), Ls.begin() + Ls.size() / 2, Ls.end());
@@ -1951,11 +1953,18 @@ TuneKey tune_key(int device, int nen, const std::vector<DomDev>& doms, const std
   int64_t kept = 0;
   for (float v : svox) kept += v != 0.0f;
   const double frac = svox.empty() ? 0.0 : (double)kept / (double)svox.size();
-  return TuneKey{device, nen, (int)std::lround(4.0 * std::log2(std::max(lmed, 1))), frac < 0.15 ? 0 : frac < 0.30 ? 1 : 2};
+  // SIMT CTAs (three groups of load cases a tile or column) on 148 SMs that hold two of them, or one (HEX20)
+  const int64_t ctas = 3 * (nen == 20 ? W.nbi : W.ntw), wave = nen == 20 ? 148 : 2 * 148;
+  return TuneKey{device,
+                 nen,
+                 (int)std::lround(4.0 * std::log2(std::max(lmed, 1))),
+                 frac < 0.15 ? 0 : frac < 0.30 ? 1 : 2,
+                 nen == 20 ? (int)std::lround(std::log2(std::max(W.layers, 1))) : W.len,
+                 ctas <= wave ? 0 : ctas <= 4 * wave ? 1 : 2};
 }
 
-// The fine-level operator of an FP32 multigrid solve, chosen per device, element type and size
-// class (median domain edge in quarter octaves, kept-voxel fraction below 0.15 / 0.30 / above)
+// The fine-level operator of an FP32 multigrid solve, chosen per device, element type, size class
+// (median domain edge in quarter octaves, kept-voxel fraction below 0.15 / 0.30 / above) and launch
 // by CUDA-event timings on the batch's own tiles and vectors:
 //  * HEX08: the SIMT sweep or the tcgen05 sweep (timed on the post-smoothing sweep);
 //  * HEX20: the SIMT column kernel or the tcgen05 brick kernel (the operator of the residual and
@@ -1963,7 +1972,7 @@ TuneKey tune_key(int device, int nen, const std::vector<DomDev>& doms, const std
 int autotune_sweep(DeviceSolver::Impl& I, SolverStats& st, Work& W, MgDev& M, const std::vector<DomDev>& doms,
                    const std::vector<float>& svox, int nen, std::string& msg) {
   cudaStream_t s = I.stream;
-  const TuneKey key = tune_key(I.device, nen, doms, svox);
+  const TuneKey key = tune_key(I.device, nen, W, doms, svox);
   auto adopt = [&](const TuneResult& r) {
     I.tensor_matvec = r.pick == 1;
     record_tuning(st, r);
