@@ -37,9 +37,14 @@ constexpr int kGramPart = 6 * 64; // upper triangle of 8 x 8 tiles of a 24 x 24 
 // A basis is made orthonormal again when a pivot of its scaled Gram matrix falls below this; 1e2 needs
 // 1 to 5 of these per solve, 1e4 lets rounding errors cost iterations.
 constexpr double kBlkRenorm = 1e-2;
-// Scaled pivots below these count as dependent columns.  C: the columns left out stay in the residual, for
-// the next refinement step.  G: below the rounding noise of FP32 directions.
-constexpr double kBlkDropC = 1e-10, kBlkDropG = 1e-7;
+// Scaled pivots below these count as dependent columns.  C: the rounding of an FP32 V-cycle leaves pivots of
+// dependent columns at up to +-3.5e-6 instead of 0, and a column of noise spoils those eliminated after it; the columns
+// left out stay in the residual, for the next refinement step.  G: below the rounding noise of FP32 directions.
+// H, the measured p.r of columns just made orthonormal, is the identity up to noise: what is not near 1 is noise.
+// Over 4608 domains of 15^3 to 56^3, bone fraction 0.05 to 0.45: at 1e-10 for C and 1e-7 for H two small bones in
+// a corner of their domain, whose load cases span 18 dimensions, took 3313 and 4625 iterations (now 27 and 24);
+// 1e-10 and 0.1 27.8 on average and 126 at most, 1e-6 and 0.1 27.2 and 126, 1e-5 27.3 with more refinement steps.
+constexpr double kBlkDropC = 1e-6, kBlkDropG = 1e-7, kBlkDropH = 0.1;
 // A column made orthonormal whose measured p.r is below this (it should be 1) is rounding noise.
 constexpr double kBlkNoise = 0.25;
 
@@ -130,8 +135,8 @@ __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
 // Both matrices are symmetric in exact arithmetic; the upper triangle of 8 x 8 tiles is computed.  In the
 // step after R <- R tau, kBlkCurv also computes H = P^T R tau and takes it in place of C = 1: tau magnifies
 // the rounding of nearly dependent columns, some of which are then nothing else.  With H the step is the
-// projection on the directions as they are, and columns whose diagonal entry shows them to be noise are left
-// out of it.
+// projection on the directions as they are, and columns whose diagonal entry or pivot shows them to be noise are
+// left out of it.
 // Bound by the FP64 tensor pipe and by reading the two blocks: 201 us on 384 domains of 32^3 (3.2 TB/s
 // while all are active).  8 warps and pieces of 256 nodes keep the atomic traffic below a tenth of
 // the reads; smaller pieces are cut when the batch would not fill the card.
@@ -270,9 +275,10 @@ __global__ void __launch_bounds__(256) k_blk_gram(const Chunk* __restrict__ chun
         if (!good) A[e] = 0.0;
       }
       __syncthreads();
-      blk_factor(Hs, U, L, T, kBlkDropG, minp, kept);
+      blk_factor(Hs, U, L, T, kBlkDropH, minp, kept);
       for (int e = tid; e < kBlkM; e += 256) {
         const int i = e / kNLC, j = e % kNLC;
+        if (T[i * (kNLC + 1)] == 0.0 || T[j * (kNLC + 1)] == 0.0) A[e] = 0.0;
         double s = 0.0;
         for (int k = 0; k < kNLC; ++k) s = fma(T[i * kNLC + k], T[j * kNLC + k], s);
         st.Cinv[e] = s;
