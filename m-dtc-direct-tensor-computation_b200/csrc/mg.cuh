@@ -349,14 +349,14 @@ __global__ void __launch_bounds__(kTailThreads, 1)
   const DomDev& C = doms_c[dom];
   const int tid = threadIdx.x, n0 = F.n[0], n1 = F.n[1], n2 = F.n[2];
   const int64_t node_off = F.node_off;
-  const float scale = (float)F.scale;
+  const double scale = F.scale;
   auto at = [](int x, int y, int zz) { return (x + kTailN * (y + kTailN * zz)) * 3 * kTailLc; };
   for (int i = tid; i < 2 * kTailVec; i += NT) src[i] = 0.f;
   for (int i = tid; i < kTailCoarse; i += NT) zc[i] = 0.f;
   for (int i = tid; i < 512; i += NT) {
     const int x = i % 8, y = i / 8 % 8, zz = i / 64;
     sv[i] = x < n0 - 1 && y < n1 - 1 && zz < n2 - 1
-                ? scale * __ldg(svox + F.vox_off + x + (int64_t)(n0 - 1) * (y + (int64_t)(n1 - 1) * zz)) : 0.f;
+                ? __ldg(svox + F.vox_off + x + (int64_t)(n0 - 1) * (y + (int64_t)(n1 - 1) * zz)) : 0.f;
   }
   for (int i = tid; i < kMgDenseN * kMgDenseN; i += NT) sm[i] = __ldg(minv + (int64_t)dom * kMgDenseN * kMgDenseN + i);
   for (int i = tid; i < kNodes; i += NT) {
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kTailThreads, 1)
     nodes([&](int n, int i, int x, int y, int zz, int k) {
       float r[3], v[3];
       tail_apply(kh, src + k, sv + (x - 1) + 8 * (y - 1) + 64 * (zz - 1), r);
-      for (int c = 0; c < 3; ++c) r[c] = sb[3 * i + c] - r[c];
+      for (int c = 0; c < 3; ++c) r[c] = sb[3 * i + c] - (float)(scale * (double)r[c]);   // the scale in FP64, as the sweeps
       if (step == turn) {
         for (int c = 0; c < 3; ++c) dst[k + c * kTailLc] = r[c];
         return;
