@@ -111,6 +111,13 @@ int64_t device_bytes_per_node(const dtc_options& o) {
   return 72 * (4 * 8 + 4 * 4) + 64 + (o.macro_order == 2 && o.tensor_estimator == 1 ? 2 * 72 * 8 : 0);
 }
 
+// and per domain, which counts where domains are small: macro forces and column states (order 2: the Gram matrix of
+// three column passes), and with the multigrid inner solve its dense coarsest level and the block CG's state
+int64_t device_bytes_per_domain(const dtc_options& o) {
+  const bool mg = o.precision == DTC_PREC_MIXED && o.inner_precond == 2;
+  return 16 * 1024 + (o.macro_order == 2 ? 72 * 72 * 8 : 0) + (mg ? kMgDomainBytes : 0);
+}
+
 }  // namespace
 
 namespace dtc {
@@ -299,7 +306,8 @@ dtc_status dtc_solve_batch(dtc_handle* h, const dtc_domain_in* in, int64_t n, dt
     for (int64_t k = 0; k < n; ++k) {
       const dtc_domain_in& d = in[k];
       const int mg = d.elem_type == DTC_HEX20 ? 2 : 1;   // HEX20 nodes live on the doubled grid
-      const double nb = (double)(mg * d.L[0] + 1) * (mg * d.L[1] + 1) * (mg * d.L[2] + 1) * device_bytes_per_node(h->opt);
+      const double nb = (double)(mg * d.L[0] + 1) * (mg * d.L[1] + 1) * (mg * d.L[2] + 1) * device_bytes_per_node(h->opt) +
+                        device_bytes_per_domain(h->opt);
       const int64_t cnt = k - cuts.back();
       const bool full = (h->opt.chunk_domains > 0 && cnt >= h->opt.chunk_domains) ||
                         (pipe > 0 && cuts.size() == 1 && cnt >= pipe);

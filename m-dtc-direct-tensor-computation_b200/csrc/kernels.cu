@@ -2470,6 +2470,8 @@ int solve_nen(DeviceSolver::Impl& I, SolverStats& stats_, std::vector<DomainTask
         (e = ensure(I, bMgList, sizeof(int) * std::max<size_t>(mgp.lists.size(), 1), msg)) ||
         (e = ensure(I, bMgNodes, sizeof(int64_t) * std::max<size_t>(mgp.nodes_l.size(), 1), msg)))
       return e;
+    static_assert(sizeof(float) * kMgDenseN * kMgDenseN + sizeof(BlkState) + sizeof(BlkCoef) +
+                          sizeof(double) * (kGramPart + kBlkM) <= kMgDomainBytes, "what the passes are cut by");
     if ((e = ensure(I, bNChunk, sizeof(int) * ndom, msg)) || (e = ensure(I, bBlkSt, sizeof(BlkState) * ndom, msg)) ||
         (e = ensure(I, bBlkCf, sizeof(BlkCoef) * ndom, msg)) ||
         (e = ensure(I, bGram, sizeof(double) * (kGramPart + kBlkM) * ndom, msg)) ||

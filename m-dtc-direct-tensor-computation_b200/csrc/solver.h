@@ -103,6 +103,10 @@ struct HostBatchDeleter {
 };
 using HostBatchPtr = std::unique_ptr<HostBatch, HostBatchDeleter>;
 
+// Device bytes of a domain in the multigrid inner solve beside its nodes: the dense inverse of the coarsest level
+// and the block CG's state.
+constexpr int64_t kMgDomainBytes = 64 * 1024;
+
 class DeviceSolver {
  public:
   struct Impl;  // device buffers and stream (kernels.cu)
