@@ -33,8 +33,7 @@ LADDER = [float(f"{m}e-{k}") for k in range(3, 10) for m in (5, 3, 2, 1)][3:]
 # the host-only reference arm cannot calibrate itself
 REF_RTOL = 5e-7
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic byte of the fine
-# sweeps, measured on 16 domains of 32^3 (profiles/k_sweep_f32_16x32cubed.md; below 1 where part of the input
-# vector was still in L2)
+# sweeps, measured on 16 domains of 32^3 (below 1 where part of the input vector was still in L2)
 DRAM_PER_ALGORITHMIC_BYTE = {"matvec_f32": 0.44, "mg_residual_f32": 0.93, "mg_postsmooth_f32": 0.99}
 # FP32 SIMT FMA peak, nominal: 148 SMs x 128 lanes x 2 flop x 1.965 GHz (the sweeps run on the
 # FMA pipe, not on tensor cores; the measured peaks cover HBM and bf16 tensor only)
@@ -646,9 +645,8 @@ def main():
                                     "frac": 40 * st["dof_iterations"] / (step_ms / 1e3) / 1e9 / peak},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": traffic, "peak_source": src,
-                             "traffic_source": (f"ncu dram bytes / algorithmic bytes = {ratio} on the 16x32^3 case "
-                                                "(profiles/k_sweep_f32_16x32cubed.md), scaled to this "
-                                                "launch" if ratio else None),
+                             "traffic_source": (f"ncu dram bytes / algorithmic bytes = {ratio} on 16 domains of 32^3, "
+                                                "scaled to this launch" if ratio else None),
                              "kernel": top, "avg_launch_us": t_launch * 1e6,
                              "flops_per_launch": kt["flops_per_launch"],
                              "achieved_tflops": kt["flops_per_launch"] / t_launch / 1e12,

@@ -64,10 +64,13 @@ typedef struct dtc_options {
   double rtol;             /* relative tolerance on ||D^-1 r|| / ||D^-1 b|| per load case;
                               the reference's PETSc option -ksp_rtol (f-src/mod_parameters.f90:31) */
   int64_t max_it;          /* CG iteration cap per load case (-ksp_max_it, :32); for the mixed
-                              path the cap on the summed inner iterations */
-  double inner_rtol;       /* mixed path: reduction asked of each FP32 inner solve
-                              (0 -> max(0.3 rtol, 1e-7)); with inner_precond = 2 of the natural
-                              norm sqrt(r . V r), V the V-cycle */
+                              path the cap on each inner solve, of which there are up to
+                              max_refine */
+  double inner_rtol;       /* mixed path: reduction asked of each FP32 inner solve.  inner_precond
+                              0 and 1: 0 -> max(0.3 rtol, 1e-7), and no further than half the
+                              absolute tolerance.  inner_precond = 2: 0 -> 1e-7, of the natural
+                              norm sqrt(r . V r), V the V-cycle, and no further than 0.3 (first
+                              inner solve) or 0.05 (later ones) of what would reach the tolerance */
   int32_t max_refine;      /* mixed path: cap on FP64 refinement steps (0 -> 12) */
   int32_t rotation_search; /* 1: run the CR1/CR2 rotation search (mod_struct_calcmat.f90:533-1603) */
   int32_t device;          /* CUDA device ordinal */

@@ -568,8 +568,7 @@ __global__ void __launch_bounds__(192) k_blk_direction(const Chunk* __restrict__
   }
 }
 
-// Iterations and failures of an inner block solve in the outer state of its load cases; clears the state
-// of the domains for the next one.
+// Iterations and failures of an inner block solve in the outer state of its load cases.
 __global__ void k_blk_finish(ColState* __restrict__ ost, const BlkState* __restrict__ state, int64_t ncol) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= ncol || !ost[i].active) return;

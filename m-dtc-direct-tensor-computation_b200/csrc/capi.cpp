@@ -137,7 +137,7 @@ void dtc_default_options(dtc_options* opt) {
   opt->precision = DTC_PREC_FP64;
   opt->rtol = 1e-3;       // -ksp_rtol 1.e-03 (f-src/mod_parameters.f90:31)
   opt->max_it = 500000;   // -ksp_max_it 500000 (:32)
-  opt->inner_rtol = 0.0;   // automatic: max(0.3 rtol, 1e-7)
+  opt->inner_rtol = 0.0;   // automatic (dtc.h)
   opt->max_refine = 12;
   opt->rotation_search = 1;
   opt->inner_precond = 1;

@@ -921,8 +921,8 @@ int allow_all_hex20(std::string& msg) {
   return allow_hex20_smem<double, true, false>(msg);
 }
 
-// Work lists of one solve: node tiles (vector kernels and the HEX08 node-centric operator)
-// and voxel columns (HEX20 operator), over the interior / all nodes.
+// Work lists of one solve: node tiles (setup and node-local kernels, the FP64 CG of tile_cg.cuh), the HEX08 sweeps'
+// tiles and voxel columns (HEX20 operator), over the interior / all nodes.
 struct Work {
   const Tile *ti, *ta, *bi, *ba;
   int64_t nti, nta, nbi, nba;
@@ -1052,7 +1052,7 @@ struct MgPlan {
   float omega0 = 0.f;                               // damping on the fine level (HEX08 or HEX20)
   std::vector<DomDev> doms;                         // nlev * ndom, level-major
   std::vector<Tile> tiles;
-  std::vector<int64_t> sm_off, sm_n, in_off, in_n, all_off, all_n;
+  std::vector<int64_t> sm_off, sm_n, all_off, all_n;
   std::vector<int64_t> sw_off, sw_n;                // smoothing tiles of the HEX08 sweeps
   std::vector<int> sw_len;                          // their nodes in x
   std::vector<int> lists;
@@ -1248,7 +1248,7 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
   struct Level {
     DomDev C;
     std::vector<float> sv;
-    std::vector<Tile> t_in, t_sm, t_all, t_sw;
+    std::vector<Tile> t_sm, t_all, t_sw;
     std::vector<int32_t> n_in;   // active interior nodes (index inside the level's grid)
   };
   std::vector<std::vector<Level>> lev(ndom);
@@ -1295,14 +1295,12 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
               if (act[x + (size_t)nx * (y + (size_t)ny * z)]) return true;
         return false;
       };
-      for (int z0 = 1; z0 <= nz - 2; z0 += kTileZ)
-        for (int y0 = 1; y0 <= ny - 2; y0 += kTileY)
-          for (int x0 = 1; x0 <= nx - 2; x0 += kTileX)
-            if (any(x0, y0, z0, 1, nx - 2, ny - 2, nz - 2)) {
-              const Tile t{d, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0};
-              Lv.t_in.push_back(t);
-              if (nlev[d] > l + 1 + P.tail) Lv.t_sm.push_back(t);
-            }
+      if (nlev[d] > l + 1 + P.tail)
+        for (int z0 = 1; z0 <= nz - 2; z0 += kTileZ)
+          for (int y0 = 1; y0 <= ny - 2; y0 += kTileY)
+            for (int x0 = 1; x0 <= nx - 2; x0 += kTileX)
+              if (any(x0, y0, z0, 1, nx - 2, ny - 2, nz - 2))
+                Lv.t_sm.push_back(Tile{d, (int16_t)x0, (int16_t)y0, (int16_t)z0, 0});
       for (int z0 = 0; z0 <= nz - 1; z0 += kTileZ)
         for (int y0 = 0; y0 <= ny - 1; y0 += kTileY)
           for (int x0 = 0; x0 <= nx - 1; x0 += kTileX)
@@ -1332,7 +1330,7 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
   // concatenate in domain order
   P.nlev = nl;
   P.doms.assign((size_t)nl * ndom, DomDev{});
-  P.sm_off.assign(nl, 0); P.sm_n.assign(nl, 0); P.in_off.assign(nl, 0); P.in_n.assign(nl, 0);
+  P.sm_off.assign(nl, 0); P.sm_n.assign(nl, 0);
   P.sw_off.assign(nl, 0); P.sw_n.assign(nl, 0);
   P.all_off.assign(nl, 0); P.all_n.assign(nl, 0); P.list_off.assign(nl, 0); P.list_n.assign(nl, 0);
   P.nl_off.assign(nl, 0); P.nl_n.assign(nl, 0); P.ns_off.assign(nl, 0); P.ns_n.assign(nl, 0);
@@ -1361,7 +1359,6 @@ void build_mg(MgPlan& P, const std::vector<DomDev>& doms0, const std::vector<flo
       cnt = (int64_t)P.tiles.size() - off;
     };
     append(&Level::t_sm, P.sm_off[l], P.sm_n[l]);
-    append(&Level::t_in, P.in_off[l], P.in_n[l]);
     append(&Level::t_all, P.all_off[l], P.all_n[l]);
     append(&Level::t_sw, P.sw_off[l], P.sw_n[l]);
     auto append_nodes = [&](auto&& takes, int64_t& off, int64_t& cnt) {
@@ -1622,7 +1619,7 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   cudaStream_t s = I.stream;
   static const MgPlan kNoLevels;
   const MgPlan& P = M ? *M->P : kNoLevels;
-  const int nseg = 7 + 6 * P.nlev;
+  const int nseg = 7 + 5 * P.nlev;
   int e;
   if ((e = ensure(I, bCompactCnt, sizeof(int) * nseg, msg))) return e;
   if ((e = ensure(I, bTilesIc, sizeof(Tile) * std::max<int64_t>(W.nti, 1), msg))) return e;
@@ -1655,12 +1652,11 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
   launch_compact(W.bt, W.nbt, act, bt, cnt + 5, s);
   launch_compact(W.tf, W.ntf, act, fc, cnt + 6, s);
   for (int l = 0; l < P.nlev; ++l) {
-    launch_compact(M->tiles + P.sm_off[l], P.sm_n[l], act, mt + P.sm_off[l], cnt + 7 + 6 * l, s);
-    launch_compact(M->tiles + P.in_off[l], P.in_n[l], act, mt + P.in_off[l], cnt + 8 + 6 * l, s);
-    launch_compact(M->lists + P.list_off[l], P.list_n[l], act, ml + P.list_off[l], cnt + 9 + 6 * l, s);
-    launch_compact(M->nodes + P.nl_off[l], P.nl_n[l], act, mn + P.nl_off[l], cnt + 10 + 6 * l, s);
-    launch_compact(M->tiles + P.sw_off[l], P.sw_n[l], act, mt + P.sw_off[l], cnt + 11 + 6 * l, s);
-    launch_compact(M->nodes + P.ns_off[l], P.ns_n[l], act, mn + P.ns_off[l], cnt + 12 + 6 * l, s);
+    launch_compact(M->tiles + P.sm_off[l], P.sm_n[l], act, mt + P.sm_off[l], cnt + 7 + 5 * l, s);
+    launch_compact(M->lists + P.list_off[l], P.list_n[l], act, ml + P.list_off[l], cnt + 8 + 5 * l, s);
+    launch_compact(M->nodes + P.nl_off[l], P.nl_n[l], act, mn + P.nl_off[l], cnt + 9 + 5 * l, s);
+    launch_compact(M->tiles + P.sw_off[l], P.sw_n[l], act, mt + P.sw_off[l], cnt + 10 + 5 * l, s);
+    launch_compact(M->nodes + P.ns_off[l], P.ns_n[l], act, mn + P.ns_off[l], cnt + 11 + 5 * l, s);
   }
   launches += nseg;
   if ((e = launch_check(msg))) return e;
@@ -1682,12 +1678,11 @@ int compact_lists(DeviceSolver::Impl& I, const Work& W, const MgDev* M, const in
     Mc->lists = ml;
     Mc->nodes = mn;
     for (int l = 0; l < P.nlev; ++l) {
-      Pc->sm_n[l] = h[7 + 6 * l];
-      Pc->in_n[l] = h[8 + 6 * l];
-      Pc->list_n[l] = h[9 + 6 * l];
-      Pc->nl_n[l] = h[10 + 6 * l];
-      Pc->sw_n[l] = h[11 + 6 * l];
-      Pc->ns_n[l] = h[12 + 6 * l];
+      Pc->sm_n[l] = h[7 + 5 * l];
+      Pc->list_n[l] = h[8 + 5 * l];
+      Pc->nl_n[l] = h[9 + 5 * l];
+      Pc->sw_n[l] = h[10 + 5 * l];
+      Pc->ns_n[l] = h[11 + 5 * l];
     }
   }
   return DTC_OK;
@@ -1801,7 +1796,7 @@ int run_cg_mg(DeviceSolver::Impl& I, int ndom, int nactive, const Work& W, const
   Work Wc = W;
   MgPlan Pc;   // offsets and counts of the multigrid lists (no bulk data)
   Pc.nlev = M.P->nlev; Pc.omega = M.P->omega; Pc.omega0 = M.P->omega0;
-  Pc.sm_off = M.P->sm_off; Pc.sm_n = M.P->sm_n; Pc.in_off = M.P->in_off; Pc.in_n = M.P->in_n;
+  Pc.sm_off = M.P->sm_off; Pc.sm_n = M.P->sm_n;
   Pc.sw_off = M.P->sw_off; Pc.sw_n = M.P->sw_n; Pc.sw_len = M.P->sw_len;
   Pc.list_off = M.P->list_off; Pc.list_n = M.P->list_n;
   Pc.nl_off = M.P->nl_off; Pc.nl_n = M.P->nl_n;

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kMgCoarseThreads) k_mg_coarse(const int* __res
 // level smooths twice) launches of a few microseconds, each a serial chain over a grid too small for the card.
 // A thread applies K to one node and load case from the differences to its 26 neighbours, which keeps
 // rigid translations exact null vectors.  Bound by shared-memory reads (81 a node and load case) and the
-// latency between its 7 (11) barriers.  One domain of 16^3: coarse levels 1.34 -> 0.71 ms of a solve, the solve
+// latency between its 7 (9) barriers.  One domain of 16^3: coarse levels 1.34 -> 0.71 ms of a solve, the solve
 // 4.7 -> 3.6 ms; 16 domains of 32^3 with 60 load cases 32 -> 23 ms, the solve 148 -> 115.
 constexpr int kTailThreads = 512, kTailLc = 4, kTailN = 9, kTailIn = 7;   // nodes per edge, interior ones
 constexpr int kTailVec = kTailN * kTailN * kTailN * 3 * kTailLc;

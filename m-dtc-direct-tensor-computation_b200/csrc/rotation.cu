@@ -182,7 +182,7 @@ __device__ __forceinline__ ArgMin block_argmin(ArgMin m, ArgMin* sh) {
 // 1-degree sweep: a thread evaluates the angles of one segment about one axis, whose normalisation (a square
 // root and three divisions) it does once.  The CTA first evaluates a coarse subset of the same grid: the
 // smallest values there bound what a candidate may reach, and the bounds shrink as its threads find better ones.
-// Bound by the FP64 pipe (80 % busy at 12 warps an SM; the register file holds no more): 66 us a tensor when there
+// Bound by the FP64 pipe (80 % busy at 12 warps an SM; the register file holds no more): 62 us a tensor when there
 // are many, 4.00 ms for 64; one CTA row of angles per thread without the bounds took 6.32.  A single tensor is
 // spread over every SM twice over: 0.10 ms, 0.24 with 64 CTAs.
 __global__ void __launch_bounds__(kSweepThreadsRot, 3) k_rot_sweep(const double* __restrict__ ee,

@@ -4,7 +4,7 @@
 // cube is mirror symmetric, so a displacement component couples only to those of the same parity under the
 // three reflections, in eight classes of three.  Per class the matrix has one or two distinct entries,
 // 8 numbers in all for any Poisson ratio (hadamard_entries), and the three translations drop out, which
-// also makes them exact.  72 additions each way and 33 products replace 576 multiply-adds per voxel and
+// also makes them exact.  72 additions each way and 31 products replace 576 multiply-adds per voxel and
 // load case, and most of the additions are shared: along x by a thread that walks a voxel row (the
 // y/z-transformed node plane between two voxels serves both), and the transform back in y and z is done
 // once per node plane.
@@ -68,7 +68,7 @@ template <> struct Lane<float> {
   static __device__ __forceinline__ V coef(V w, float s) { return __fmul2_rn(w, make_float2(s, s)); }
   static __device__ __forceinline__ V load(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
   static __device__ __forceinline__ void store(float* p, V v) { *reinterpret_cast<float2*>(p) = v; }
-  // v * scale with the FP64 scale as two floats: within one rounding of the product
+  // v * scale with the FP64 scale as two floats: the float that the product in FP64 rounds to (4 million pairs)
   struct Scale {
     float2 hi, lo;
     __device__ __forceinline__ explicit Scale(double s) {
@@ -220,7 +220,8 @@ enum { kSwApply = 0, kSwApplyDot = 1, kSwRes = 2, kSwPost = 3 };
 // bytes of load cases).  Node planes are staged through a ring in shared memory two steps ahead of
 // their use (each value once per CTA, from four voxel rows), the voxel factors for the whole tile at the
 // start, with a bit mask of the kept voxels per row that says who has work, what to stage and whose share
-// a node row gets.  16 warps per SM (126 registers; budgets that spill, for 18 or more warps, were slower).
+// a node row gets.  16 warps per SM (122 to 128 registers, none spilled).  A first form with register budgets for 18
+// warps spilled, ended in an illegal memory access twice, for a cause not found, and was left out.
 // Bound by instruction issue (49 %) and the barrier per plane, DRAM at 13 %.  Average over the launches of a
 // solve of 64 domains of 32^3, against the node-centric sweeps that applied the 24 x 24 matrix: residual
 // 361 -> 249 us, post-smoothing 375 -> 298, CG application 319 -> 224; FP64 application, 27 x 20^3,
