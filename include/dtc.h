@@ -70,7 +70,8 @@ typedef struct dtc_options {
                               0 and 1: 0 -> max(0.3 rtol, 1e-7), and no further than half the
                               absolute tolerance.  inner_precond = 2: 0 -> 1e-7, of the natural
                               norm sqrt(r . V r), V the V-cycle, and no further than 0.3 (first
-                              inner solve) or 0.05 (later ones) of what would reach the tolerance */
+                              inner solve) or 0.05 (second; then a quarter of the one before)
+                              of what would reach the tolerance */
   int32_t max_refine;      /* mixed path: cap on FP64 refinement steps (0 -> 12) */
   int32_t rotation_search; /* 1: run the CR1/CR2 rotation search (mod_struct_calcmat.f90:533-1603) */
   int32_t device;          /* CUDA device ordinal */
@@ -90,7 +91,8 @@ typedef struct dtc_options {
                               PCJACOBI), 1 = node-block Jacobi (3x3 diagonal blocks),
                               2 = multigrid V-cycle on halved voxel grids (HEX20 domains are
                               first coarsened to the HEX08 mesh of the same voxels); the load
-                              cases of a domain then share one Krylov space (block CG) */
+                              cases of a domain then share one Krylov space (block CG); from the
+                              sixth refinement step on as 1 */
   int32_t tensor_estimator; /* how ff is formed from the solutions: 0 = projection of the
                               reaction forces (the reference, mod_struct_calcmat.f90:254-280),
                               error linear in the solve error; 1 = energy products
