@@ -242,11 +242,11 @@ __global__ void __launch_bounds__(kThreads) k_boundary_values(const Tile* __rest
   const bool rowok = yy >= 1 && yy <= D.n[1] - 2 && zz >= 1 && zz <= D.n[2] - 2; \
   const int64_t col = (int64_t)t.dom * kNLC + lc;
 
-// CG vector kernels of the Jacobi paths over pieces of one domain's active interior nodes: a thread owns 16 bytes
-// of load cases (2 FP64, 4 FP32) and walks the nodes of its slot, so that every access is a 16-byte one and a CTA
-// reduces into one domain's dot products.  Bound by L2 and HBM: FP64, 27 x 20^3, averaged over a solve, update
-// 54 -> 36 us and direction 21 -> 20 against walking node tiles with one load case per thread, inactive nodes
-// included; 8 x 23^3 update 15 us.
+// CG vector kernels of the Jacobi paths (HEX08 in FP64 at loose tolerances: tile_cg.cuh) over pieces of one domain's
+// active interior nodes: a thread owns 16 bytes of load cases (2 FP64, 4 FP32) and walks the nodes of its slot, so
+// that every access is a 16-byte one and a CTA reduces into one domain's dot products.  Bound by L2 and HBM: FP64, 27 x
+// 20^3, averaged over a solve, update 54 -> 36 us and direction 21 -> 20 against walking node tiles with one load
+// case per thread, inactive nodes included; 8 x 23^3 update 15 us.
 template <typename T> struct Cols16;
 template <> struct Cols16<double> {
   static constexpr int kCols = 2;
@@ -951,7 +951,8 @@ const Hadamard<T>& hadamard(const DeviceSolver::Impl& I) {
 
 // One HEX08 sweep over nt tiles of len nodes in x.
 template <typename T, bool ALL, int MODE>
-void launch_sweep(int64_t nt, int len, cudaStream_t s, const DeviceSolver::Impl& I, const Tile* tiles, const DomDev* dd, const float* svox,
+void launch_sweep(int64_t nt, int len, cudaStream_t s, const DeviceSolver::Impl& I, const Tile* tiles,
+                  const DomDev* dd, const float* svox,
                   const T* u, T* y, double scale, const float* binv, const T* b, float omega, double* acc,
                   const int* act) {
   if (nt <= 0) return;
@@ -965,7 +966,8 @@ template <bool DOT>
 void launch_tile_matvec(const Work& W, const DomDev* dd, const float* svox, const double* u, double* y, double scale,
                         double* acc, const int* act, int bnd_only, cudaStream_t s) {
   if (W.ntf <= 0) return;
-  k_tile_matvec<DOT><<<(unsigned)(3 * W.ntf), kThreads, 0, s>>>(W.tf, dd, svox, W.I->kh64, u, y, scale, acc, act, bnd_only);
+  k_tile_matvec<DOT><<<(unsigned)(3 * W.ntf), kThreads, 0, s>>>(W.tf, dd, svox, W.I->kh64, u, y, scale, acc, act,
+                                                                bnd_only);
 }
 
 template <typename T, bool ALL, int MODE>

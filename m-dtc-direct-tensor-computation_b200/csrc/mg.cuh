@@ -330,8 +330,9 @@ __device__ __forceinline__ void tail_apply(const VoxelMatrix<float>& kh, const f
 __global__ void __launch_bounds__(kTailThreads, 1)
     k_mg_tail(const int* __restrict__ list, const DomDev* __restrict__ doms_f, const DomDev* __restrict__ doms_c,
               const float* __restrict__ svox, const __grid_constant__ VoxelMatrix<float> kh,
-              const uint8_t* __restrict__ flags, const float* __restrict__ binv, const float* __restrict__ minv, const float* __restrict__ b, float* __restrict__ z, float omega,
-              int steps, const int* __restrict__ dom_active) {
+              const uint8_t* __restrict__ flags, const float* __restrict__ binv, const float* __restrict__ minv,
+              const float* __restrict__ b, float* __restrict__ z, float omega, int steps,
+              const int* __restrict__ dom_active) {
   extern __shared__ __align__(16) unsigned char tail_smem[];
   constexpr int kNodes = kTailItems / kTailLc, NT = kTailThreads;
   float* src = reinterpret_cast<float*>(tail_smem);

@@ -9,8 +9,8 @@
 // fewer the results are the same bit for bit from run to run.
 //
 // The price, against the sweeps and the list kernels (sweep.cuh, k_update): 8 domains of 23^3 at rtol 1e-3
-// 12.8 -> 22.6 ms.  At kTightRtol and below the stop no longer shows (two runs differ by less than 1e-9 of the
-// tensor), and the faster kernels are used.
+// 12.7 -> 22.9 ms (operator 32 -> 60 us, update 13 -> 23, direction 10 -> 13).  At kTightRtol and below the stop no
+// longer shows (two runs differ by less than 1e-9 of the tensor), and the faster kernels are used.
 #pragma once
 
 namespace dtc {
@@ -23,8 +23,8 @@ constexpr double kTightRtol = 1e-10;
 // corners' values from u, kb being the index of the row's value at plane x for its load case, and adds to node x
 // (corner offset 0 in x) and node x+1 (offset 1).  FIRST: only node x+1 belongs to the tile.
 template <bool FIRST>
-__device__ __forceinline__ void voxel_rd(const VoxelMatrix<double>& kh, const double* __restrict__ u, int64_t kb, int sy, int sz, int b, int c,
-                                         float s, double (&cur)[3], double (&nxt)[3]) {
+__device__ __forceinline__ void voxel_rd(const VoxelMatrix<double>& kh, const double* __restrict__ u, int64_t kb,
+                                         int sy, int sz, int b, int c, float s, double (&cur)[3], double (&nxt)[3]) {
   const int l0 = corner_local(0, 1 - b, 1 - c), l1 = corner_local(1, 1 - b, 1 - c);
   double t0 = 0, t1 = 0, t2 = 0, q0 = 0, q1 = 0, q2 = 0;
 #pragma unroll 1
